@@ -648,6 +648,12 @@ __global__ void __launch_bounds__(REL_TX * REL_TY) k_reliable_vec(Geom g, double
       const double m = out[0] * s->inv_nfluid;
       s->rshift = m;
       const double rr = fmax(out[1] - out[0] * m, 0.0);
+      // The FP32 increment's rounding (about 6e-8 diag |x|, so for a smooth
+      // pressure that grows with N^2) can leave the true residual far above
+      // the recursive one.  The old direction then belongs to another
+      // residual, and beta = rz_new / rz would carry it on for hundreds of
+      // iterations: PCG starts again from the true residual.
+      if (rr > 1.5 * s->rr) s->first = 1;
       s->rr = rr;
       s->rr_anchor = rr;
       s->rmax = out[2];
