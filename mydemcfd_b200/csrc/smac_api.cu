@@ -100,6 +100,8 @@ enum CoefType { CT_F64 = 0, CT_F32 = 1, CT_BF16 = 2 };
 struct Level {
   Geom g{};
   int cx = 0, cy = 0, cz = 0;  // coarsened from the grid above
+  CoarseAxis ax{}, ay{}, az{};  // distance factors of its faces (k_coarsen_coeffs)
+  double wx = 1.0, wy = 1.0, wz = 1.0;  // width of the last cell per axis, in regular cells
   double *bx64 = nullptr, *by64 = nullptr, *bz64 = nullptr;  // stencil weights f_b / h^2 of this grid
   double *x64 = nullptr, *x64b = nullptr, *rhs64 = nullptr;  // levels >= 1 (two iterates: out-of-place sweeps)
   void *bxm = nullptr, *bym = nullptr, *bzm = nullptr;  // mixed-precision weights
@@ -122,11 +124,13 @@ struct smac_handle {
   int nlev = 0;
   int lc = 0;  // first grid of the single-CTA coarse set
   // the cluster set (k_coarse_cluster): its first grid (-1: not used), grids
-  // spread over the ranks, and per grid its chunk and shared-memory offsets
-  int lk = -1, kc_nd = 0;
-  int kc_chunk[MAXL] = {}, kc_off[MAXL][5] = {};
-  int kc_elems = 0;
-  bool kc_ok[2] = {false, false};  // [FP32, FP64]: launchable
+  // spread over the ranks, per grid its chunk and shared-memory offsets
+  // (one per precision: [FP32, FP64])
+  struct ClusterPlan {
+    int lk = -1, nd = 0;
+    int chunk[MAXL] = {}, off[MAXL][5] = {};
+    int elems = 0;
+  } kc[2];
   Level lv[MAXL];
   uint8_t* fluid = nullptr;   // padded cell bits: 1 C_INTERIOR, 2 fluid unknown
   double *fbx = nullptr, *fby = nullptr, *fbz = nullptr;  // masked f_b, padded (divergence, correction, adjoint)
@@ -496,16 +500,17 @@ void launch_update(smac_handle* h, const Geom& g, T* x, const T* d, T* r, const 
 // Whether the lower part of the V-cycle runs in the cluster kernel, and the
 // first grid of the part that does not run sweep by sweep.
 bool use_cluster(const smac_handle* h, bool mixed) {
-  return h->lk >= 1 && h->opts.coarse_kernel == SMAC_COARSE_AUTO && h->kc_ok[mixed ? 0 : 1];
+  return h->opts.coarse_kernel == SMAC_COARSE_AUTO && h->kc[mixed ? 0 : 1].lk >= 1;
 }
-int coarse_start(const smac_handle* h, bool mixed) { return use_cluster(h, mixed) ? h->lk : h->lc; }
+int coarse_start(const smac_handle* h, bool mixed) { return use_cluster(h, mixed) ? h->kc[mixed ? 0 : 1].lk : h->lc; }
 
 // Global bytes of the cluster kernel per launch: the first grid's rhs in and
 // x out, every grid's three weight arrays in.
 double cluster_bytes(const smac_handle* h, bool mixed) {
   const double s = mixed ? 4.0 : 8.0;
-  double b = 2.0 * s * (double)h->lv[h->lk].g.cells();
-  for (int l = h->lk; l < h->nlev; ++l) {
+  const int lk = h->kc[mixed ? 0 : 1].lk;
+  double b = 2.0 * s * (double)h->lv[lk].g.cells();
+  for (int l = lk; l < h->nlev; ++l) {
     const double sc = mixed ? 4.0 : 8.0;  // (BF16 weights through their FP32 copies)
     b += 3.0 * sc * (double)h->lv[l].g.cells();
   }
@@ -514,17 +519,18 @@ double cluster_bytes(const smac_handle* h, bool mixed) {
 
 template <class T>
 void launch_cluster(smac_handle* h, bool mixed, const T* rhs, T* x) {
+  const auto& P = h->kc[mixed ? 0 : 1];
   ClusterSet set{};
-  set.n = h->nlev - h->lk;
-  set.nd = h->kc_nd;
+  set.n = h->nlev - P.lk;
+  set.nd = P.nd;
   for (int q = 0; q < set.n; ++q) {
-    const Level& L = h->lv[h->lk + q];
+    const Level& L = h->lv[P.lk + q];
     ClusterLevel& C = set.L[q];
     C.g = L.g;
     C.cx = L.cx; C.cy = L.cy; C.cz = L.cz;
-    C.chunk = h->kc_chunk[q];
-    C.ox = h->kc_off[q][0]; C.orhs = h->kc_off[q][1];
-    C.obx = h->kc_off[q][2]; C.oby = h->kc_off[q][3]; C.obz = h->kc_off[q][4];
+    C.chunk = P.chunk[q];
+    C.ox = P.off[q][0]; C.orhs = P.off[q][1];
+    C.obx = P.off[q][2]; C.oby = P.off[q][3]; C.obz = P.off[q][4];
     // every array staged as T: BF16 weights through their exact FP32 copies
     const bool wide = mixed && L.ctm == CT_BF16;
     C.ctype = mixed ? CT_F32 : CT_F64;
@@ -534,7 +540,7 @@ void launch_cluster(smac_handle* h, bool mixed, const T* rhs, T* x) {
   }
   set.rhs0 = rhs;
   set.x0 = x;
-  launch_pdl(k_coarse_cluster<T>, KCL, kcl_threads<T>(), (size_t)h->kc_elems * sizeof(T), h->stream, set, h->opts.nu1,
+  launch_pdl(k_coarse_cluster<T>, KCL, kcl_threads<T>(), (size_t)P.elems * sizeof(T), h->stream, set, h->opts.nu1,
       h->opts.nu2, h->opts.coarse_sweeps, (const Scalars*)h->s);
   h->alg_bytes += cluster_bytes(h, mixed);
   h->launches += 1;
@@ -577,10 +583,12 @@ smac_status launch_vcycle(smac_handle* h, T* r0, T* z0a, T* z0b, bool mixed, boo
     CKL();
     const Level& Lc = h->lv[l + 1];
     auto S = stencil<T, CS>(g, CF(l, 0), CF(l, 1), CF(l, 2));
-    if (std::is_same<T, CS>::value && Lc.cx && Lc.cy && Lc.cz)
-      launch_pdl(k_resid_restrict2<T>, grid_planes(Lc.g.nx, Lc.g.ny, Lc.g.nz), kBlock, 0, h->stream, g, cur[l], B(l),
+    if (std::is_same<T, CS>::value && Lc.cx && Lc.cy && Lc.cz) {
+      const bool odd = (g.nx | g.ny | g.nz) & 1;
+      launch_pdl(odd ? k_resid_restrict2<T, true> : k_resid_restrict2<T, false>,
+          grid_planes(Lc.g.nx, Lc.g.ny, Lc.g.nz), kBlock, 0, h->stream, g, cur[l], B(l),
           sh, stencil<T, T>(g, CF(l, 0), CF(l, 1), CF(l, 2)), Lc.g, B(l + 1), h->s);
-    else
+    } else
       launch_pdl(k_resid_restrict<T, CS>, grid_planes(Lc.g.nx, Lc.g.ny, Lc.g.nz), kBlock, 0, h->stream, g, cur[l], B(l),
           sh, S, Lc.g, Lc.cx, Lc.cy, Lc.cz, B(l + 1), h->s);
     account(h, g, 2 * s + 3 * sc + s / 8, 1);
@@ -901,12 +909,9 @@ bool cluster_attr(int bytes) {
   return n >= 1;
 }
 
-void setup_cluster(smac_handle* h, int smem_optin) {
-  h->lk = -1;
-  int lk = -1;
-  for (int l = 1; l < h->nlev; ++l)
-    if (h->lv[l].g.cells() <= KCL_TOP) { lk = l; break; }
-  if (lk < 1 || h->lv[h->nlev - 1].g.cells() > KCL_SOLO || h->nlev - lk > MAX_CLL) return;
+template <class T>
+bool plan_cluster(smac_handle* h, int lk, int smem_optin) {
+  auto& P = h->kc[sizeof(T) == 8 ? 1 : 0];
   const int n = h->nlev - lk;
   int nd = 0;
   while (nd < n && h->lv[lk + nd].g.cells() > KCL_SOLO) ++nd;
@@ -922,21 +927,36 @@ void setup_cluster(smac_handle* h, int smem_optin) {
     const Geom& g = h->lv[lk + q].g;
     if (q > 0 && q < nd && h->lv[lk + q].cz) chunk /= 2;
     const int c = q < nd ? chunk : g.nz;
-    if (c < 1) return;
-    h->kc_chunk[q] = c;
+    if (c < 1) return false;
+    P.chunk[q] = c;
     const long long nx = g.nx, ny = g.ny;
-    h->kc_off[q][0] = take(c * nx * ny);            // x
-    h->kc_off[q][1] = take(c * nx * ny);            // rhs
-    h->kc_off[q][2] = take(c * ny * (nx + 1));      // bx
-    h->kc_off[q][3] = take(c * (ny + 1) * nx);      // by
-    h->kc_off[q][4] = take((c + 1) * ny * nx);      // bz
+    P.off[q][0] = take(c * nx * ny);            // x
+    P.off[q][1] = take(c * nx * ny);            // rhs
+    P.off[q][2] = take(c * ny * (nx + 1));      // bx
+    P.off[q][3] = take(c * (ny + 1) * nx);      // by
+    P.off[q][4] = take((c + 1) * ny * nx);      // bz
+    if (tot * (int)sizeof(T) > smem_optin) return false;
   }
-  if (tot * 8 > (1LL << 30)) return;
-  h->kc_elems = (int)tot;
-  h->kc_nd = nd;
-  h->kc_ok[0] = tot * 4 <= smem_optin && cluster_attr<float>((int)(tot * 4));
-  h->kc_ok[1] = tot * 8 <= smem_optin && cluster_attr<double>((int)(tot * 8));
-  if (h->kc_ok[0] || h->kc_ok[1]) h->lk = lk;
+  if (!cluster_attr<T>((int)(tot * (int)sizeof(T)))) return false;
+  P.elems = (int)tot;
+  P.nd = nd;
+  P.lk = lk;
+  return true;
+}
+
+// Per precision the first grid from which the set fits: the chunks of a grid
+// whose planes do not divide evenly are rounded up, and FP64 takes twice the
+// shared memory, so a grid of <= KCL_TOP cells may not.  (No grid past the
+// single-CTA set's first: the weights of that set may be BF16, which the
+// separately launched sweeps of the grids above do not read.)
+void setup_cluster(smac_handle* h, int smem_optin) {
+  if (h->lv[h->nlev - 1].g.cells() > KCL_SOLO) return;
+  bool ok32 = false, ok64 = false;
+  for (int l = 1; l <= h->lc; ++l) {
+    if (h->lv[l].g.cells() > KCL_TOP || h->nlev - l > MAX_CLL) continue;
+    ok32 = ok32 || plan_cluster<float>(h, l, smem_optin);
+    ok64 = ok64 || plan_cluster<double>(h, l, smem_optin);
+  }
 }
 
 // Tensor maps for every separately launched grid, or use_tma = false.
@@ -1054,20 +1074,28 @@ smac_status smac_create(const smac_grid_desc* desc, const smac_options* opts, vo
     memcpy(g_err, keep, sizeof(keep));
     return st;
   };
-  // hierarchy: halve a direction while it stays even and >= min_coarse
+  // hierarchy: halve a direction while the result stays >= min_coarse, an odd
+  // extent n to (n + 1) / 2 (k_coarsen_coeffs).  Stopping a direction at its
+  // first odd extent left a coarsest grid of up to the whole problem to one
+  // CTA and a few sweeps: 150 x 100 x 75 took 58 iterations and 120 ms,
+  // 99^3 64 and 848 ms (mixed).
   {
     int nx = desc->nx, ny = desc->ny, nz = desc->nz;
     double ix2 = 1.0 / (desc->dx * desc->dx), iy2 = 1.0 / (desc->dy * desc->dy), iz2 = 1.0 / (desc->dz * desc->dz);
     h->lv[0].g = make_geom(nx, ny, nz, ix2, iy2, iz2);
     h->nlev = 1;
     while (h->nlev < o.max_levels && is_gmg(o)) {
-      const int cx = (nx % 2 == 0 && nx / 2 >= o.min_coarse), cy = (ny % 2 == 0 && ny / 2 >= o.min_coarse),
-                cz = (nz % 2 == 0 && nz / 2 >= o.min_coarse);
+      const int cx = (nx + 1) / 2 >= o.min_coarse, cy = (ny + 1) / 2 >= o.min_coarse,
+                cz = (nz + 1) / 2 >= o.min_coarse;
       if (!cx && !cy && !cz) break;
-      if (cx) { nx /= 2; ix2 *= 0.25; }
-      if (cy) { ny /= 2; iy2 *= 0.25; }
-      if (cz) { nz /= 2; iz2 *= 0.25; }
       Level& L = h->lv[h->nlev];
+      const Level& F = h->lv[h->nlev - 1];
+      L.ax = coarse_axis(cx, nx, F.wx, &L.wx);
+      L.ay = coarse_axis(cy, ny, F.wy, &L.wy);
+      L.az = coarse_axis(cz, nz, F.wz, &L.wz);
+      if (cx) { nx = (nx + 1) / 2; ix2 *= 0.25; }
+      if (cy) { ny = (ny + 1) / 2; iy2 *= 0.25; }
+      if (cz) { nz = (nz + 1) / 2; iz2 *= 0.25; }
       L.g = make_geom(nx, ny, nz, ix2, iy2, iz2);
       L.cx = cx; L.cy = cy; L.cz = cz;
       h->nlev += 1;
@@ -1233,8 +1261,9 @@ smac_status smac_set_coefficients(smac_handle* h, const double* fbx, const doubl
     Level& F = h->lv[l - 1];
     Level& L = h->lv[l];
     const dim3 gr = grid_planes(L.g.nx + 1, L.g.ny + 1, L.g.nz + 1);
-    k_coarsen_coeffs<double><<<gr, kBlock, 0, h->stream>>>(F.g, L.g, L.cx, L.cy, L.cz, F.bx64, F.by64, F.bz64, L.bx64,
-                                                           L.by64, L.bz64, nullptr, nullptr, nullptr);
+    k_coarsen_coeffs<double><<<gr, kBlock, 0, h->stream>>>(F.g, L.g, L.cx, L.cy, L.cz, L.ax, L.ay, L.az, F.bx64,
+                                                           F.by64, F.bz64, L.bx64, L.by64, L.bz64, nullptr, nullptr,
+                                                           nullptr);
     CKL();
     const long long n = L.g.alloc;
     if (L.ctm == CT_BF16) {

@@ -273,8 +273,9 @@ __device__ __noinline__ void cl_resid_restrict(ClusterView<T> V, ClGrid L, ClGri
     for (int dk = 0; dk < rz; ++dk)
       for (int dj = 0; dj < ry; ++dj)
         for (int di = 0; di < rx; ++di) {
-          const int k = (Lc.cz ? 2 * K : K) + dk;
-          cl_resid_add(V, L, (Lc.cx ? 2 * I : I) + di, (Lc.cy ? 2 * J : J) + dj, k, k - k0, np, acc);
+          const int i = (Lc.cx ? 2 * I : I) + di, j = (Lc.cy ? 2 * J : J) + dj, k = (Lc.cz ? 2 * K : K) + dk;
+          if (i >= L.nx || j >= L.ny || k >= L.nz) continue;  // no such child (odd extent)
+          cl_resid_add(V, L, i, j, k, k - k0, np, acc);
         }
     *V.rhsp(Lc, I, J, K) = (T)Ar<A>::div(acc, (A)(rx * ry * rz));
   }

@@ -108,10 +108,35 @@ __global__ void __launch_bounds__(TNT) k_fluid_finalize(Geom g, const double* __
 // coarse face (2x2 in 3-D), times 1/4 when the face-normal direction is
 // coarsened (1/H^2 = (1/h^2)/4, G_GMGSolver.cu:71-73,135-137); computed in
 // FP64 and stored as C.  Both scalings are powers of two, so they are exact.
+//
+// An odd extent n is halved to (n + 1) / 2: its last coarse cell has one child
+// and half the width.  In units of the grid's regular cell let the last cell
+// of an axis be l wide (1 on the finest grid), and L on the coarse grid:
+// L = (1 + l) / 2 for even n, l / 2 for odd n.  The equations of every grid
+// are finite volumes divided by the regular cell's volume, so a face's weight
+// is its area over the distance of its two cells: the sum over the children
+// that exist, still divided by 4, gives the area, and CoarseAxis the ratio of
+// the distances for the face in front of the last cell and for the wall
+// (1/4 where both cells are regular).  Restriction then is the sum of the
+// children's residuals over 8, also where children are missing: the transpose
+// of the prolongation, so the V-cycle stays symmetric.
+struct CoarseAxis {
+  double regular, last, wall;  // factors of faces I < n-1, I = n-1, I = n
+};
+inline CoarseAxis coarse_axis(bool halved, int n_fine, double l, double* L) {
+  if (!halved) { *L = l; return CoarseAxis{1.0, 1.0, 1.0}; }
+  const bool odd = n_fine & 1;
+  *L = odd ? 0.5 * l : 0.5 * (1.0 + l);
+  return CoarseAxis{0.25, 0.25 * (1.0 + (odd ? l : 1.0)) / (1.0 + *L), 0.25 * l / *L};
+}
+__device__ __forceinline__ double coarse_factor(const CoarseAxis& a, int I, int nc) {
+  return I < nc - 1 ? a.regular : I == nc - 1 ? a.last : a.wall;
+}
 template <class C>
-__global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, const double* __restrict__ fbx,
-                                 const double* __restrict__ fby, const double* __restrict__ fbz, C* bx, C* by,
-                                 C* bz, double* bx64, double* by64, double* bz64) {
+__global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, CoarseAxis ax, CoarseAxis ay, CoarseAxis az,
+                                 const double* __restrict__ fbx, const double* __restrict__ fby,
+                                 const double* __restrict__ fbz, C* bx, C* by, C* bz, double* bx64, double* by64,
+                                 double* bz64) {
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = blockIdx.y * blockDim.y + threadIdx.y;
   const int K = blockIdx.z;
@@ -119,29 +144,32 @@ __global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, const
   const int c = gc.idx(I, J, K);
   const int ry = cy ? 2 : 1, rz = cz ? 2 : 1, rx = cx ? 2 : 1;
   if (J < gc.ny && K < gc.nz) {  // x-face I
-    const int i = cx ? 2 * I : I;
+    const int i = cx ? min(2 * I, gf.nx) : I, j0 = cy ? 2 * J : J, k0 = cz ? 2 * K : K;
     double s = 0.0;
     for (int dk = 0; dk < rz; ++dk)
-      for (int dj = 0; dj < ry; ++dj) s += fbx[gf.idx(i, (cy ? 2 * J : J) + dj, (cz ? 2 * K : K) + dk)];
-    s *= (cx ? 0.25 : 1.0) / (double)(ry * rz);
+      for (int dj = 0; dj < ry; ++dj)
+        if (j0 + dj < gf.ny && k0 + dk < gf.nz) s += fbx[gf.idx(i, j0 + dj, k0 + dk)];
+    s *= coarse_factor(ax, I, gc.nx) / (double)(ry * rz);
     bx[c] = coef_from_double<C>(s);
     if (bx64) bx64[c] = s;
   }
   if (I < gc.nx && K < gc.nz) {  // y-face J
-    const int jj = cy ? 2 * J : J;
+    const int jj = cy ? min(2 * J, gf.ny) : J, i0 = cx ? 2 * I : I, k0 = cz ? 2 * K : K;
     double s = 0.0;
     for (int dk = 0; dk < rz; ++dk)
-      for (int di = 0; di < rx; ++di) s += fby[gf.idx((cx ? 2 * I : I) + di, jj, (cz ? 2 * K : K) + dk)];
-    s *= (cy ? 0.25 : 1.0) / (double)(rx * rz);
+      for (int di = 0; di < rx; ++di)
+        if (i0 + di < gf.nx && k0 + dk < gf.nz) s += fby[gf.idx(i0 + di, jj, k0 + dk)];
+    s *= coarse_factor(ay, J, gc.ny) / (double)(rx * rz);
     by[c] = coef_from_double<C>(s);
     if (by64) by64[c] = s;
   }
   if (I < gc.nx && J < gc.ny) {  // z-face K
-    const int kk = cz ? 2 * K : K;
+    const int kk = cz ? min(2 * K, gf.nz) : K, i0 = cx ? 2 * I : I, j0 = cy ? 2 * J : J;
     double s = 0.0;
     for (int dj = 0; dj < ry; ++dj)
-      for (int di = 0; di < rx; ++di) s += fbz[gf.idx((cx ? 2 * I : I) + di, (cy ? 2 * J : J) + dj, kk)];
-    s *= (cz ? 0.25 : 1.0) / (double)(rx * ry);
+      for (int di = 0; di < rx; ++di)
+        if (i0 + di < gf.nx && j0 + dj < gf.ny) s += fbz[gf.idx(i0 + di, j0 + dj, kk)];
+    s *= coarse_factor(az, K, gc.nz) / (double)(rx * ry);
     bz[c] = coef_from_double<C>(s);
     if (bz64) bz64[c] = s;
   }
@@ -879,6 +907,7 @@ __global__ void __launch_bounds__(TNT) k_resid_restrict(Geom g, const T* __restr
     for (int dj = 0; dj < ry; ++dj)
       for (int di = 0; di < rx; ++di) {
         const int i = (cx ? 2 * I : I) + di, j = (cy ? 2 * J : J) + dj, k = (cz ? 2 * K : K) + dk;
+        if (i >= g.nx || j >= g.ny || k >= g.nz) continue;  // no such child (odd extent)
         const int c = g.idx(i, j, k);
         A wxm, wxp, wym, wyp, wzm, wzp;
         S.coeffs(c, g.px, g.ps, wxm, wxp, wym, wyp, wzm, wzp);
@@ -895,8 +924,9 @@ __global__ void __launch_bounds__(TNT) k_resid_restrict(Geom g, const T* __restr
 // The same for a coarse grid halved in every direction: each thread reads its
 // 2x2x2 block's rows, the rows and planes around it and the faces once, as
 // 2-vectors of cells (i = 2I, 2I+1), and sums the eight residuals in the
-// order of k_resid_restrict.
-template <class T>
+// order of k_resid_restrict.  ODD: some extent is odd, so the last block along
+// it lacks children; what lies beyond the pad row or plane is not read.
+template <class T, bool ODD>
 __global__ void __launch_bounds__(TNT) k_resid_restrict2(Geom g, const T* __restrict__ x, const T* __restrict__ rhs,
                                                          const double* shift, Stencil<T, T> S, Geom gc, T* rhs_c,
                                                          const Scalars* s) {
@@ -915,34 +945,40 @@ __global__ void __launch_bounds__(TNT) k_resid_restrict2(Geom g, const T* __rest
     a = (A)v.x;
     b = (A)v.y;
   };
+  const bool i1 = !ODD || i + 1 < g.nx, j1 = !ODD || j + 1 < g.ny, k1 = !ODD || k + 1 < g.nz;
   // x: rows j-1 .. j+2 on planes k, k+1; planes k-1, k+2 on rows j, j+1
   A xr[2][4][2], xz[2][2][2], xl[2][2], xh[2][2];
 #pragma unroll
   for (int dk = 0; dk < 2; ++dk) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) ld2(x, g.idx(i, j - 1 + r, k + dk), xr[dk][r][0], xr[dk][r][1]);
+    for (int r = 0; r < 4; ++r) {
+      xr[dk][r][0] = xr[dk][r][1] = (A)0;
+      if (r < 3 || j1) ld2(x, g.idx(i, j - 1 + r, k + dk), xr[dk][r][0], xr[dk][r][1]);
+    }
 #pragma unroll
     for (int dj = 0; dj < 2; ++dj) {
       const int c = g.idx(i, j + dj, k + dk);
       xl[dk][dj] = (A)x[c - 1];
-      xh[dk][dj] = (A)x[c + 2];
+      xh[dk][dj] = i1 ? (A)x[c + 2] : (A)0;
     }
   }
 #pragma unroll
   for (int dj = 0; dj < 2; ++dj) {
+    xz[1][dj][0] = xz[1][dj][1] = (A)0;
     ld2(x, g.idx(i, j + dj, k - 1), xz[0][dj][0], xz[0][dj][1]);
-    ld2(x, g.idx(i, j + dj, k + 2), xz[1][dj][0], xz[1][dj][1]);
+    if (k1) ld2(x, g.idx(i, j + dj, k + 2), xz[1][dj][0], xz[1][dj][1]);
   }
   A acc = (A)0;
 #pragma unroll
   for (int dk = 0; dk < 2; ++dk) {
 #pragma unroll
     for (int dj = 0; dj < 2; ++dj) {
+      if (ODD && ((dj && !j1) || (dk && !k1))) continue;
       const int c = g.idx(i, j + dj, k + dk);
       A b0, b1, bx0, bx1, by0, by1, bu0, bu1, bz0, bz1, bw0, bw1;
       ld2(rhs, c, b0, b1);
       ld2(S.bx, c, bx0, bx1);
-      const A bx2 = (A)S.bx[c + 2];
+      const A bx2 = i1 ? (A)S.bx[c + 2] : (A)0;
       ld2(S.by, c, by0, by1);
       ld2(S.by, c + g.px, bu0, bu1);
       ld2(S.bz, c, bz0, bz1);
@@ -953,6 +989,7 @@ __global__ void __launch_bounds__(TNT) k_resid_restrict2(Geom g, const T* __rest
       const A* row = xr[dk][1 + dj];
 #pragma unroll
       for (int di = 0; di < 2; ++di) {
+        if (ODD && di && !i1) continue;
         const A wxm = di ? bx1 : bx0, wxp = di ? bx2 : bx1;
         const A wym = di ? by1 : by0, wyp = di ? bu1 : bu0;
         const A wzm = di ? bz1 : bz0, wzp = di ? bw1 : bw0;
@@ -1050,6 +1087,7 @@ __device__ __forceinline__ void cta_resid_restrict(const CoarseLevel& L, const C
       for (int dj = 0; dj < ry; ++dj)
         for (int di = 0; di < rx; ++di) {
           const int i = (Lc.cx ? 2 * I : I) + di, j = (Lc.cy ? 2 * J : J) + dj, k = (Lc.cz ? 2 * K : K) + dk;
+          if (i >= g.nx || j >= g.ny || k >= g.nz) continue;  // no such child (odd extent)
           const int c = g.idx(i, j, k);
           A wxm, wxp, wym, wyp, wzm, wzp;
           S.coeffs(c, g.px, g.ps, wxm, wxp, wym, wyp, wzm, wzp);

@@ -193,6 +193,9 @@ __global__ void __launch_bounds__(TmaTile<T>::NT, 2)
     };
     const int j = j0 + jr, ip = i0 + 2 * m;
 
+    // The prolongation from a grid halved in every direction, of even extents
+    // (behind an odd extent's last cell the parent is not a coarse ghost).
+    const bool pro4 = MODE == 2 && cx && cy && cz && !((g.nx | g.ny | g.nz) & 1);
     // Colour c0 at tile column xcol (xin tile coordinates: cell i = i0 - 4 + xcol)
     // and tile row jt (cell j = j0 - 1 + jt) of plane k; zero outside the domain.
     auto red_at = [&](int xcol, int jt, int k, const unsigned char* sm, const unsigned char* s0,
@@ -219,8 +222,8 @@ __global__ void __launch_bounds__(TmaTile<T>::NT, 2)
         A n4 = (A)Xm[cp], n5 = (A)Xp[cp];
         if constexpr (MODE == 2) {
           // prolongation of the coarse correction, added to each neighbour
-          if (cx && cy && cz) {
-            // Halved in every direction: three neighbours share the cell's
+          if (pro4) {
+            // Even extents, all halved: three neighbours share the cell's
             // coarse parent, the other three are the parent's neighbours
             // on the side the cell's parity selects.  A neighbour outside
             // the domain maps to a coarse ghost, which holds 0, like the
@@ -247,10 +250,9 @@ __global__ void __launch_bounds__(TmaTile<T>::NT, 2)
       }
     };
 
-    // Coarse values of a fine cell (MODE 2 on a grid halved in every
-    // direction), loaded from L2 one step before the cell's update so that
-    // the loads overlap the barrier and the colour-(1-c0) pass.
-    const bool pro4 = MODE == 2 && cx && cy && cz;
+    // Coarse values of a fine cell (MODE 2, pro4), loaded from L2 one step
+    // before the cell's update so that the loads overlap the barrier and the
+    // colour-(1-c0) pass.
     auto coarse4 = [&](int ia, int ja, int k) -> Coarse4<A> {
       Coarse4<A> q{(A)0, (A)0, (A)0, (A)0};
       if (pro4 && (unsigned)ia < (unsigned)g.nx && (unsigned)ja < (unsigned)g.ny && (unsigned)k < (unsigned)g.nz) {
