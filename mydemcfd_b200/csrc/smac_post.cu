@@ -29,6 +29,7 @@
 // a ghost cell whose source cell is C_SOLID computes that cell's new value
 // itself (from interior neighbours that nothing writes), and a corner face
 // computes its two ghost neighbours' values itself.
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 
@@ -734,9 +735,8 @@ __global__ void __launch_bounds__(256) k_st_rim(StArgs A) {
 // Offsets into the predictor's and the mass flux's arrays are 32-bit: a grid
 // must keep every array below 2^31 entries (index_fits).  That bound is not a
 // practical limit here: the predictor's two dozen FP64 input arrays of a grid
-// that large would need more than 400 GB.  32-bit offsets cut the kernel's
-// registers and spills (80 instead of 164 bytes of spill stores) and its time
-// at 256^3 from 3.31 to 3.14 ms.
+// that large would need more than 400 GB.  32-bit offsets keep the kernels'
+// registers down.
 struct MomArgs {
   int N[3];
   const uint8_t* ft[3];
@@ -941,48 +941,245 @@ __device__ __forceinline__ double m_vstar(const MomArgs& A, const int* b) {
   return DMUL(DSUB(1.0, A.sf[AF] ? A.sf[AF][f] : 0.0), vs);
 }
 
-// One thread per face index (x, y) of plane z of the box 1..N+1;
-// blockIdx.z takes SMAC_PV_ZG planes of family 0, the same planes of
-// family 1, then of family 2, so that the three families of a few planes run
-// together and share the arrays they all read (velocities, fluxes, cell
-// fields) through L2, while an SM mostly runs one family's code at a time.
-// At 256^3, groups of 1, 2, 4, 8 and 16 planes: 2.268, 2.239, 2.244, 2.307
-// and 2.523 ms (two-way 2.540, 2.497, 2.507, 2.608, 2.839).  Only
-// F_INTERIOR faces are written.  The kernel waits on chains of dependent
-// loads (a face type, then the value it selects), so resident warps matter
-// more than registers: 5 blocks per SM (48 registers,
-// a few spills to L1) measured 3.32 ms at 256^3 with 64-bit offsets (3.14 ms
-// with the 32-bit ones now used), against 3.60 ms with 4 blocks, 4.27 ms
-// with 3 and 3.43 ms with 6.  Family-major block order (all
-// planes of one family, then the next, so that resident warps share one
-// family's code) took 3.64 ms: the interleaved families' shared reads
-// through L2 are worth more than the instruction-cache locality.  Block
-// shapes of 256 faces at 256^3: 32 x 8 2.28 ms, 64 x 4 2.32, 16 x 16 2.37,
-// 128 x 2 2.50 (two-way 2.56, 2.62, 2.65, 2.85).
-#ifndef SMAC_PV_BX
-#define SMAC_PV_BX 32  // predictor block: SMAC_PV_BX x (256 / SMAC_PV_BX) faces of one plane
-#endif
-#ifndef SMAC_PV_ZG
-#define SMAC_PV_ZG 2  // planes per family group: blockIdx.z runs G planes of family 0, then of 1, then of 2
-#endif
-constexpr int kPvBx = SMAC_PV_BX, kPvBy = 256 / SMAC_PV_BX, kPvZg = SMAC_PV_ZG;
-static_assert(kPvBx * kPvBy == 256, "the predictor's block has 256 threads");
-template <bool TW>
-__global__ void __launch_bounds__(256, 5) k_predict_vstar(MomArgs A) {
-  const int q = blockIdx.z % (3 * kPvZg);
-  const int fam = q / kPvZg;
-  const int z = blockIdx.z / (3 * kPvZg) * kPvZg + q % kPvZg + 1;
-  const int x = blockIdx.x * kPvBx + threadIdx.x + 1, y = blockIdx.y * kPvBy + threadIdx.y + 1;
-  if (x > A.N[0] + 1 || y > A.N[1] + 1 || z > A.N[2] + 1) return;
+// The predictor kernel.  A face is regular when every face of the three
+// families within two indices of it is F_INTERIOR (so nothing it reads passes
+// through a boundary rule); all but a shell of the box and around solids are.
+// For regular faces u* is a sum of differences of side terms, the stress and
+// the convective flux through the control volume's sides, and a minus side's
+// terms are the plus side's of the neighbour bit for bit (the same products
+// and sums of the same values: the limiter's arguments, the flux's sign and
+// the edge means coincide).  So a block takes one family's faces of a tile of
+// 31 x 8 indices and a chunk of planes, finds the regular ones from the types
+// (read once per chunk), marches them in z without a type or a branch
+// (m_march), and evaluates the rest from a queue with the boundary rules
+// (m_vstar), all lanes busy.
+//
+// Measured at 256^3 (a two-phase step's fields): 1.60 ms; before, with every
+// face evaluating both sides and a type loaded beside each value, 2.34 ms,
+// bound by dependent loads and instruction misses.  It is now bound by the
+// latency of the march's loads, of which 43% hit L1, at the 32 warps per SM
+// that 64 registers allow (46% of the issue slots, 22% of the FP64 pipe; the
+// queue is 0.25 ms of it).  Not kept: blocks of 3 or 5 per SM (1.90, 1.69);
+// chunks of 6, 8 or 14 planes (1.57, 1.57, 1.70; 192^3 likes 10: 1.24 against
+// 1.29, 1.27, 1.28 for its whole explicit half); a group of warps per family
+// in one block, so that the arrays come through L1 once (1.70 to 1.82); one
+// thread per index for the three families, marching over planes staged in
+// shared memory by 8-byte asynchronous copies, the y-sides exchanged there
+// (2.05: 16 warps per SM and a barrier per plane); the same reading through
+// L1 (2.58); prefetches into L1 or L2 a plane ahead (1.58).
+constexpr int PV_X = 31, PV_Y = 8, PV_NT = 32 * PV_Y, PV_ZMAX = 10, PV_BLOCKS = 4;
+constexpr int PV_FC = 36, PV_FR = PV_Y + 4;  // the type tile: columns x0-2 .. x0+33, rows y0-2 .. y0+PV_Y+1
+static_assert(PV_ZMAX + 4 <= 32 && PV_ZMAX * PV_Y * 32 <= 65536, "plane bits and 16-bit queue entries");
+
+// MUSCL/minmod flux through the side between v0 and np (the values before and
+// after them along the axis: nm and far); f is the advecting flux.
+__device__ __forceinline__ double m_side_flux(double f, double nm, double v0, double np, double far) {
+  const double d = DSUB(np, v0);
+  const bool up = f > 0.0;
+  const double s = m_minmod(up ? d : DSUB(far, np), up ? DSUB(v0, nm) : d);
+  return DMUL(f, DADD(up ? v0 : np, DMUL(f < 0.0 ? -0.5 : 0.5, s)));
+}
+__device__ __forceinline__ double m_mean(double a, double b) { return DMUL(0.5, DADD(a, b)); }
+
+// Advecting flux through the plus side along D of the family-AF face with
+// indices b; zp: the step to plane z+1 (0 behind the last one).
+template <int AF, int D>
+__device__ __forceinline__ double m_adv(const MomArgs& A, const int* b, int zp) {
+  const int sd = D == 2 ? zp * A.st[D][2] : A.st[D][D];
+  if (D == AF) return m_mean(__ldg(A.mf[AF] + (b[AF])), __ldg(A.mf[AF] + (b[AF] + sd)));
+  const int qd = b[D] + sd;
+  return m_mean(__ldg(A.mf[D] + (qd - A.st[D][AF])), __ldg(A.mf[D] + (qd)));
+}
+// Stress on that side; v0, np: the face's value and its neighbour's.
+template <int AF, int D, bool TW>
+__device__ __forceinline__ double m_tau(const MomArgs& A, const int* b, int zp, double v0, double np) {
+  if (D == AF) {
+    const double t = DMUL(__ldg(A.mu + (b[3])), DSUB(np, v0));
+    return TW ? DMUL(__ldg(A.eps_old + (b[3])), t) : t;
+  }
+  const int qd = b[D] + (D == 2 ? zp * A.st[D][2] : A.st[D][D]), qda = qd - A.st[D][AF];
+  const double mu = m_mean(__ldg(A.muf[D] + (qd)), __ldg(A.muf[D] + (qda)));
+  const double t = DMUL(mu, DADD(DMUL(DSUB(__ldg(A.v[D] + (qd)), __ldg(A.v[D] + (qda))), A.ih[AF]), DMUL(DSUB(np, v0), A.ih[D])));
+  if (!TW) return t;
+  const int c = b[3], cm = c - A.st[3][AF], sd = D == 2 ? zp * A.st[3][2] : A.st[3][D];
+  const double* e = A.eps_old;
+  const double sum = D > AF ? DADD(DADD(DADD(__ldg(e + (cm)), __ldg(e + (c))), __ldg(e + (cm + sd))), __ldg(e + (c + sd)))
+                            : DADD(DADD(DADD(__ldg(e + (cm)), __ldg(e + (cm + sd))), __ldg(e + (c))), __ldg(e + (c + sd)));
+  return DMUL(DMUL(0.25, sum), t);
+}
+
+// The march of one family: a thread takes the face at its (x, y) of planes
+// z0 .. z1-1 and writes it where the bit of `regular` for the plane is set.
+// Minus sides: x from the lane before (lane 0 is halo), z from the plane
+// before (registers), y evaluated.  Indices are clamped into the arrays;
+// clamped values reach only faces that are not regular.
+template <int AF, bool TW>
+__device__ __forceinline__ void m_march(const MomArgs& A, int x, int y, int z0, int z1, uint32_t regular) {
+  const int xl = min(max(x, 1), A.N[0] - 1), yl = min(max(y, 2), A.N[1] - 1), last = A.N[2] + 1;
   int b[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) b[k] = x * A.st[k][0] + y * A.st[k][1] + z * A.st[k][2];
+  for (int k = 0; k < 4; ++k) b[k] = xl + yl * A.st[k][1] + (z0 - 1) * A.st[k][2];
+  const double* V = A.v[AF];
+  const int sy = A.st[AF][1], sz = A.st[AF][2];
+  double vm, v0, vp, zt, zf;
+  {  // the plus z-side of plane z0 - 1 (z0 - 1 >= 0, z0 <= last)
+    const int f = b[AF];
+    vm = __ldg(V + (f - (z0 > 1 ? sz : 0)));
+    v0 = __ldg(V + (f));
+    vp = __ldg(V + (f + sz));
+    const double far = __ldg(V + (f + (z0 < last ? 2 * sz : sz)));
+    zf = m_side_flux(m_adv<AF, 2>(A, b, 1), vm, v0, vp, far);
+    zt = m_tau<AF, 2, TW>(A, b, 1, v0, vp);
+    vm = v0;
+    v0 = vp;
+    vp = far;
+  }
+  for (int z = z0; z < z1; ++z) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) b[k] += A.st[k][2];
+    const int f = b[AF], c = b[3], cm = c - A.st[3][AF], zp = z < last;
+    const double vn = __ldg(V + (f + (z + 1 < last ? 2 * sz : zp * sz)));
+    const double xm = __ldg(V + (f - 1)), xp = __ldg(V + (f + 1)), xx = __ldg(V + (f + 2));
+    const double ymm = __ldg(V + (f - 2 * sy)), ym = __ldg(V + (f - sy)), yp = __ldg(V + (f + sy)), ypp = __ldg(V + (f + 2 * sy));
+    const double inv_rho = __ldg(A.fb[AF] + (f)), rc = __ldg(A.rho_old + (c)), rm = __ldg(A.rho_old + (cm)), pc = __ldg(A.p + (c)), pm = __ldg(A.p + (cm));
+    const double fx = m_side_flux(m_adv<AF, 0>(A, b, 1), xm, v0, xp, xx);
+    const double tx = m_tau<AF, 0, TW>(A, b, 1, v0, xp);
+    const double fy = m_side_flux(m_adv<AF, 1>(A, b, 1), ym, v0, yp, ypp);
+    const double ty = m_tau<AF, 1, TW>(A, b, 1, v0, yp);
+    double fym, tym;
+    {
+      const int d[4] = {b[0] - A.st[0][1], b[1] - A.st[1][1], b[2] - A.st[2][1], b[3] - A.st[3][1]};
+      fym = m_side_flux(m_adv<AF, 1>(A, d, 1), ymm, ym, v0, yp);
+      tym = m_tau<AF, 1, TW>(A, d, 1, ym, v0);
+    }
+    const double fz = m_side_flux(m_adv<AF, 2>(A, b, zp), vm, v0, vp, vn);
+    const double tz = m_tau<AF, 2, TW>(A, b, zp, v0, vp);
+    const double fxm = __shfl_up_sync(0xffffffffu, fx, 1), txm = __shfl_up_sync(0xffffffffu, tx, 1);
+    if ((regular >> (z - z0)) & 1u) {
+      // (see m_vstar: the own axis' stress first, then the other two in axis order; convection in axis order)
+      const double dt[3] = {DSUB(tx, txm), DSUB(ty, tym), DSUB(tz, zt)};
+      double tmp = DMUL(DMUL(2.0, dt[AF]), A.ih2[AF]);
+      tmp = DADD(tmp, DMUL(dt[Others<AF>::D0], A.ih[Others<AF>::D0]));
+      tmp = DADD(tmp, DMUL(dt[Others<AF>::D1], A.ih[Others<AF>::D1]));
+      tmp = DSUB(tmp, DMUL(DSUB(fx, fxm), A.ih[0]));
+      tmp = DSUB(tmp, DMUL(DSUB(fy, fym), A.ih[1]));
+      tmp = DSUB(tmp, DMUL(DSUB(fz, zf), A.ih[2]));
+      const double rho_old_f = DMUL(0.5, DADD(rc, rm));
+      const double coupling = DMUL(A.imp[AF] ? A.imp[AF][f] : 0.0, A.inv_volume);
+      double vs;
+      if (TW) {
+        const double eo = DMUL(0.5, DADD(__ldg(A.eps_old + (cm)), __ldg(A.eps_old + (c))));
+        const double en = DMUL(0.5, DADD(__ldg(A.eps_new + (cm)), __ldg(A.eps_new + (c))));
+        tmp = DSUB(tmp, DMUL(DMUL(eo, DSUB(pc, pm)), A.ih[AF]));
+        const double ier = __ddiv_rn(inv_rho, en);
+        vs = DADD(DMUL(ier, DADD(DADD(DMUL(DMUL(eo, rho_old_f), v0), DMUL(A.dt, tmp)), coupling)),
+                  DMUL(A.dt, A.g[AF]));
+      } else {
+        tmp = DSUB(tmp, DMUL(DSUB(pc, pm), A.ih[AF]));
+        vs = DADD(DMUL(inv_rho, DADD(DMUL(v0, rho_old_f), coupling)),
+                  DMUL(A.dt, DADD(DMUL(inv_rho, tmp), A.g[AF])));
+      }
+      A.vs[AF][f] = DMUL(DSUB(1.0, A.sf[AF] ? A.sf[AF][f] : 0.0), vs);
+    }
+    vm = v0;
+    v0 = vp;
+    vp = vn;
+    zf = fz;
+    zt = tz;
+  }
+}
+
+// The indices in the block's queue, evaluated with the boundary rules.
+template <int AF, bool TW>
+__device__ __forceinline__ void m_queue(const MomArgs& A, const uint16_t* queue, int count, int x0, int y0, int z0) {
+  for (int e = threadIdx.y * 32 + threadIdx.x; e < count; e += PV_NT) {
+    const int q = queue[e];
+    const int x = x0 - 1 + (q & 31), y = y0 + (q >> 5) % PV_Y, z = z0 + q / (32 * PV_Y);
+    int b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) b[k] = x + y * A.st[k][1] + z * A.st[k][2];
+    if (A.ft[AF][b[AF]] == 0) A.vs[AF][b[AF]] = m_vstar<AF, TW>(A, b);
+  }
+}
+
+// blockIdx.z: chunk of zc planes (<= PV_ZMAX) and family, families fastest, so
+// that the three families of a chunk share the arrays they all read through
+// L2.  fast: every extent is at least 4 (else no face is regular and the
+// clamped indices would not exist).
+template <bool TW>
+__global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_vstar(const __grid_constant__ MomArgs A, int zc,
+                                                                         int fast) {
+  __shared__ uint8_t types[PV_ZMAX + 4][PV_FR * PV_FC];
+  __shared__ uint16_t queue[PV_X * PV_Y * PV_ZMAX];
+  __shared__ int qcount;
+  const int lane = threadIdx.x, row = threadIdx.y, tid = row * 32 + lane;
+  const int N0 = A.N[0], N1 = A.N[1], N2 = A.N[2];
+  const int fam = blockIdx.z % 3;
+  const int x0 = blockIdx.x * PV_X + 1, y0 = blockIdx.y * PV_Y + 1, z0 = blockIdx.z / 3 * zc + 1;
+  const int z1 = min(z0 + zc, N2 + 2);  // planes z0 .. z1-1
+  const int x = x0 - 1 + lane, y = y0 + row;
+  const bool own = lane >= 1 && x <= N0 + 1 && y <= N1 + 1;
+  if (tid == 0) qcount = 0;
+
+  // The types around the chunk, OR-ed over the families (1 outside the
+  // arrays): planes z0-2 .. z1+1.
+  bool any = false;
+  const int np = z1 - z0 + 4;
+#pragma unroll
+  for (int q = 0; q < (PV_FR * PV_FC + PV_NT - 1) / PV_NT; ++q) {
+    const int e = tid + q * PV_NT, r = e / PV_FC, gx = x0 - 2 + e - r * PV_FC, gy = y0 - 2 + r;
+    if (e >= PV_FR * PV_FC) break;
+    const bool in = gx >= 0 && gx <= N0 + 1 && gy >= 0 && gy <= N1 + 1;
+    const int o0 = gy * A.st[0][1] + gx, o1 = gy * A.st[1][1] + gx, o2 = gy * A.st[2][1] + gx;
+#pragma unroll 4
+    for (int p = 0; p < np; ++p) {
+      const int gz = z0 - 2 + p;
+      uint32_t t = 1;
+      if (in && gz >= 0 && gz <= N2 + 1)
+        t = A.ft[0][o0 + gz * A.st[0][2]] | A.ft[1][o1 + gz * A.st[1][2]] | A.ft[2][o2 + gz * A.st[2][2]];
+      types[p][e] = (uint8_t)t;
+      any |= t != 0;
+    }
+  }
+  // bit p: a type other than F_INTERIOR within two rows and columns on plane z0 - 2 + p
+  uint32_t near = 0;
+  if (__syncthreads_or(any)) {
+    for (int p = 0; p < np; ++p) {
+      uint32_t a = 0, b = 0;
+#pragma unroll
+      for (int r = 0; r < 5; ++r) {
+        a |= types[p][(row + r) * PV_FC + lane];
+        if (lane < 4) b |= types[p][(row + r) * PV_FC + 32 + lane];
+      }
+      const unsigned long long m = __ballot_sync(0xffffffffu, a != 0) |
+                                   ((unsigned long long)__ballot_sync(0xffffffffu, b != 0) << 32);
+      near |= (((m >> max(lane - 1, 0)) & 0x1f) ? 1u : 0u) << p;
+    }
+  }
+  const uint32_t planes = (1u << (z1 - z0)) - 1u;
+  const uint32_t mine = own ? planes : 0u;
+  const uint32_t regular = fast ? mine & ~(near | near >> 1 | near >> 2 | near >> 3 | near >> 4) : 0u;
+  // the others, queued: a warp takes its planes in turn
+  for (uint32_t w = __reduce_or_sync(0xffffffffu, mine & ~regular); w; w &= w - 1) {
+    const int p = __ffs(w) - 1;
+    const bool odd = ((mine & ~regular) >> p) & 1u;
+    const unsigned m = __ballot_sync(0xffffffffu, odd);
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&qcount, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (odd) queue[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)((p * PV_Y + row) * 32 + lane);
+  }
+  __syncthreads();
+  const bool march = __any_sync(0xffffffffu, regular != 0u);
   if (fam == 0) {
-    if (A.ft[0][b[0]] == 0) A.vs[0][b[0]] = m_vstar<0, TW>(A, b);
+    if (march) m_march<0, TW>(A, x, y, z0, z1, regular);
+    m_queue<0, TW>(A, queue, qcount, x0, y0, z0);
   } else if (fam == 1) {
-    if (A.ft[1][b[1]] == 0) A.vs[1][b[1]] = m_vstar<1, TW>(A, b);
+    if (march) m_march<1, TW>(A, x, y, z0, z1, regular);
+    m_queue<1, TW>(A, queue, qcount, x0, y0, z0);
   } else {
-    if (A.ft[2][b[2]] == 0) A.vs[2][b[2]] = m_vstar<2, TW>(A, b);
+    if (march) m_march<2, TW>(A, x, y, z0, z1, regular);
+    m_queue<2, TW>(A, queue, qcount, x0, y0, z0);
   }
 }
 
@@ -1513,12 +1710,23 @@ smac_status predict_vstar(const char* fn, const smac_grid_desc* d, const smac_bo
     A.st[k][2] = (int)(S0 * S1);
   }
   fill_table(&A.bc, bc);
-  const dim3 grid((unsigned)((d->nx + 1 + kPvBx - 1) / kPvBx), (unsigned)((d->ny + 1 + kPvBy - 1) / kPvBy),
-                  3u * (unsigned)((d->nz + 1 + kPvZg - 1) / kPvZg * kPvZg));
+  // planes per chunk: the fewest steps per resident block, counting a chunk's
+  // types, first side and first loads as three more
+  const int tx = (d->nx + 1 + PV_X - 1) / PV_X, ty = (d->ny + 1 + PV_Y - 1) / PV_Y, planes = d->nz + 1;
+  const long long slots = (long long)PV_BLOCKS * sm_count();
+  int zc = 1;
+  long long best = -1;
+  for (int cand = std::min(PV_ZMAX, planes); cand >= std::min(3, planes); --cand) {
+    const long long blocks = 3LL * tx * ty * ((planes + cand - 1) / cand);
+    const long long cost = ((blocks + slots - 1) / slots) * (cand + 3);
+    if (best < 0 || cost < best) { best = cost; zc = cand; }
+  }
+  const dim3 grid((unsigned)tx, (unsigned)ty, 3u * (unsigned)((planes + zc - 1) / zc)), block(32, PV_Y);
+  const int fast = d->nx >= 4 && d->ny >= 4 && d->nz >= 4;
   if (tw)
-    k_predict_vstar<true><<<grid, dim3(kPvBx, kPvBy), 0, (cudaStream_t)stream>>>(A);
+    k_predict_vstar<true><<<grid, block, 0, (cudaStream_t)stream>>>(A, zc, fast);
   else
-    k_predict_vstar<false><<<grid, dim3(kPvBx, kPvBy), 0, (cudaStream_t)stream>>>(A);
+    k_predict_vstar<false><<<grid, block, 0, (cudaStream_t)stream>>>(A, zc, fast);
   return launch_status(fn);
 }
 
