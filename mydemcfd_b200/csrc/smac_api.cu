@@ -187,7 +187,23 @@ T* base_of(const Geom& g, T* p) {
   return p - g.guard;
 }
 
-inline int kz_for(const Geom& g) { return g.nz >= 64 ? 16 : (g.nz >= 16 ? 8 : 4); }
+// Planes per block of a kernel that marches in z with bx x by blocks per
+// plane: as many as leave MARCH_BLOCKS blocks (of 128 threads) per SM.  The
+// direction kernel at 64^3 (FP32), 64 blocks of 16 planes, took 26 us.  With
+// no such bound, 4, 8, 16 and 32 blocks: mixed projection of 64^3 908, 822,
+// 821, 822, 822 us, of 150 x 100 x 75 1686, 1558, 1581, 1614, 1600; pressure
+// step of 192^3 6664, 6661, 6556, 6561, 6720; projection of 256^3 5746, 5748,
+// 5752, 5777, 5856.
+constexpr int MARCH_BLOCKS = 8;
+inline int march_kz(const smac_handle* h, const Geom& g, long long bx, long long by, int least) {
+  int kz = g.nz >= 64 ? 16 : (g.nz >= 16 ? 8 : 4);
+  while (kz > least && bx * by * ((g.nz + kz - 1) / kz) < (long long)MARCH_BLOCKS * h->num_sms) kz /= 2;
+  return kz;
+}
+// ... of one with a thread per cell (its loads come four planes at a time)
+inline int kz_for(const smac_handle* h, const Geom& g) {
+  return march_kz(h, g, (g.nx + TBX - 1) / TBX, (g.ny + TBY - 1) / TBY, 4);
+}
 inline dim3 grid_cells(const Geom& g, int kz) {
   return dim3((g.nx + TBX - 1) / TBX, (g.ny + TBY - 1) / TBY, (g.nz + kz - 1) / kz);
 }
@@ -471,7 +487,8 @@ bool launch_sweep(smac_handle* h, int l, int mode, bool dot, const T* xin, T* xo
 }
 
 // Mixed precision: the FP64 true residual and reliable update (k_reliable_vec).
-void launch_reliable(smac_handle* h, const Geom& g, const Stencil<double, double>& S64, int kz) {
+void launch_reliable(smac_handle* h, const Geom& g, const Stencil<double, double>& S64) {
+  const int kz = march_kz(h, g, (g.nx + 2 * REL_TX - 1) / (2 * REL_TX), (g.ny + REL_TY - 1) / REL_TY, 2);
   const dim3 gr((g.nx + 2 * REL_TX - 1) / (2 * REL_TX), (g.ny + REL_TY - 1) / REL_TY, (g.nz + kz - 1) / kz);
   launch_pdl(k_reliable_vec<float>, gr, dim3(REL_TX, REL_TY, 1), 0, h->stream, g, h->x64a, h->x64b, h->e32, h->b64, S64,
       h->r32, h->red, h->s, kz);
@@ -480,8 +497,9 @@ void launch_reliable(smac_handle* h, const Geom& g, const Stencil<double, double
 // d = z - zshift + beta d, q = A d, p.Ap (k_dir_matvec_vec).
 template <class T>
 void launch_dir_matvec(smac_handle* h, const Geom& g, const T* z, const T* dold, T* dnew, const Stencil<T, T>& S,
-                       T* q, int kz) {
+                       T* q) {
   constexpr int NV = Vec16<T>::n;
+  const int kz = march_kz(h, g, (g.nx + DMV_TX * NV - 1) / (DMV_TX * NV), (g.ny + DMV_TY - 1) / DMV_TY, 2);
   const dim3 gr((g.nx + DMV_TX * NV - 1) / (DMV_TX * NV), (g.ny + DMV_TY - 1) / DMV_TY, (g.nz + kz - 1) / kz);
   launch_pdl(k_dir_matvec_vec<T>, gr, dim3(DMV_TX, DMV_TY, 1), 0, h->stream, g, z, dold, dnew, S, q, h->fluid, h->red,
       h->s, kz);
@@ -647,7 +665,7 @@ smac_status launch_vcycle(smac_handle* h, T* r0, T* z0a, T* z0b, bool mixed, boo
 // `parity` selects which direction buffer is the old one.
 smac_status launch_iteration(smac_handle* h, bool mixed, bool gmg, int parity) {
   const Geom& g = h->lv[0].g;
-  const int kz = kz_for(g);
+  const int kz = kz_for(h, g);
   const dim3 gr = grid_cells(g, kz);
   const bool fused_dot = gmg && h->lc > 0;
   if (!mixed) {
@@ -667,7 +685,7 @@ smac_status launch_iteration(smac_handle* h, bool mixed, bool gmg, int parity) {
     double* dold = parity ? h->d64b : h->d64;
     double* dnew = parity ? h->d64 : h->d64b;
     auto S = stencil<double, double>(g, h->lv[0].bx64, h->lv[0].by64, h->lv[0].bz64);
-    launch_dir_matvec<double>(h, g, z, dold, dnew, S, h->q64, kz);
+    launch_dir_matvec<double>(h, g, z, dold, dnew, S, h->q64);
     launch_update<double>(h, g, h->x64a, dnew, h->r64, h->q64);
     account(h, g, 7 * 8, 1);
     account(h, g, 6 * 8, 1);
@@ -694,10 +712,10 @@ smac_status launch_iteration(smac_handle* h, bool mixed, bool gmg, int parity) {
     float* dold = parity ? h->d32b : h->d32;
     float* dnew = parity ? h->d32 : h->d32b;
     auto S = stencil<float, float>(g, h->lv[0].bxm, h->lv[0].bym, h->lv[0].bzm);
-    launch_dir_matvec<float>(h, g, z, dold, dnew, S, h->q32, kz);
+    launch_dir_matvec<float>(h, g, z, dold, dnew, S, h->q32);
     launch_update<float>(h, g, h->e32, dnew, h->r32, h->q32);
     auto S64 = stencil<double, double>(g, h->lv[0].bx64, h->lv[0].by64, h->lv[0].bz64);
-    launch_reliable(h, g, S64, kz);
+    launch_reliable(h, g, S64);
     account(h, g, 7 * 4, 1);
     account(h, g, 6 * 4, 1);
     h->launches += 1;  // the FP64 residual kernel (its bytes are counted when it runs)
@@ -1058,6 +1076,8 @@ smac_status smac_create(const smac_grid_desc* desc, const smac_options* opts, vo
   if (!h) { set_err("smac_create: out of host memory"); return SMAC_BAD_ARG; }
   h->desc = *desc;
   h->opts = o;
+  h->num_sms = prop.multiProcessorCount;
+  h->l2_bytes = prop.l2CacheSize;
   h->R = RefDims{desc->nx, desc->ny, desc->nz};
   if (cuda_stream) {
     h->stream = (cudaStream_t)cuda_stream;
@@ -1159,7 +1179,7 @@ smac_status smac_create(const smac_grid_desc* desc, const smac_options* opts, vo
   {
     long long maxb = 0;
     for (int l = 0; l < h->nlev; ++l) {
-      const dim3 gr = grid_cells(h->lv[l].g, kz_for(h->lv[l].g));
+      const dim3 gr = grid_cells(h->lv[l].g, kz_for(h, h->lv[l].g));
       maxb = std::max(maxb, (long long)gr.x * gr.y * gr.z);
       const dim3 gp = grid_planes(h->lv[l].g.nx, h->lv[l].g.ny, h->lv[l].g.nz);
       maxb = std::max(maxb, (long long)gp.x * gp.y * gp.z);
@@ -1177,8 +1197,6 @@ smac_status smac_create(const smac_grid_desc* desc, const smac_options* opts, vo
     if (eh != cudaSuccess) { set_err("cudaHostAlloc: %s", cudaGetErrorString(eh)); return fail(SMAC_CUDA_ERROR); }
     memset(h->hs, 0, sizeof(Scalars));
   }
-  h->num_sms = prop.multiProcessorCount;
-  h->l2_bytes = prop.l2CacheSize;
   setup_tma(h);
   setup_zm(h);
   setup_cluster(h, prop.sharedMemPerBlockOptin);
@@ -1246,8 +1264,8 @@ smac_status smac_set_coefficients(smac_handle* h, const double* fbx, const doubl
       g, h->R, fbx, fby, fbz, ct, fxt, fyt, fzt, h->fbx, h->fby, h->fbz, h->lv[0].bx64, h->lv[0].by64,
       h->lv[0].bz64, h->fluid);
   CKL();
-  k_fluid_finalize<<<grid_cells(g, kz_for(g)), kBlock, 0, h->stream>>>(g, h->fbx, h->fby, h->fbz, h->fluid, h->red,
-                                                                       h->s, kz_for(g));
+  k_fluid_finalize<<<grid_cells(g, kz_for(h, g)), kBlock, 0, h->stream>>>(g, h->fbx, h->fby, h->fbz, h->fluid, h->red,
+                                                                       h->s, kz_for(h, g));
   CKL();
   // FP32 fine copy for the mixed-precision Krylov operator
   {
@@ -1405,7 +1423,7 @@ smac_status run_solve(smac_handle* h, const double** xout) {
   const bool gmg = is_gmg(o);
   const bool pure = is_pure(o);
   const Geom& g = h->lv[0].g;
-  const int kz = kz_for(g);
+  const int kz = kz_for(h, g);
   const size_t bytes = sizeof(double) * (size_t)g.alloc;
   h->alg_bytes = 0.0;
   h->launches = 0;
@@ -1470,7 +1488,7 @@ smac_status run_solve(smac_handle* h, const double** xout) {
           h->hs->status = 0;
           h->hs->do_reliable = 1;
           TRY(scalars_to_device(h));
-          launch_reliable(h, g, S, kz);
+          launch_reliable(h, g, S);
           CKL();
         } else {
           launch_pdl(k_true_residual, grid_cells(g, kz), kBlock, 0, h->stream, g, h->x64a, h->b64, S, h->r64, 1, h->red,
@@ -1582,7 +1600,7 @@ smac_status export_solution(smac_handle* h, const double* x, double* p_delta) {
   const dim3 gp = grid_planes(g.nx, g.ny, g.nz);
   const bool pure = is_pure(h->opts);
   if (pure) {
-    k_sum_fluid<<<grid_cells(g, kz_for(g)), kBlock, 0, h->stream>>>(g, x, h->fluid, h->red, h->s, kz_for(g));
+    k_sum_fluid<<<grid_cells(g, kz_for(h, g)), kBlock, 0, h->stream>>>(g, x, h->fluid, h->red, h->s, kz_for(h, g));
     CKL();
   }
   constexpr int KZ = 4;
@@ -1676,7 +1694,7 @@ smac_status smac_project_adjoint(smac_handle* h, const double* gvx, const double
   TRY(run_solve(h, &x));
   account(h, g, 3 * 8 + 3 * 8 + 1 + 8, 1);
   const dim3 gp = grid_planes(g.nx, g.ny, g.nz);
-  k_sum_fluid<<<grid_cells(g, kz_for(g)), kBlock, 0, h->stream>>>(g, x, h->fluid, h->red, h->s, kz_for(g));
+  k_sum_fluid<<<grid_cells(g, kz_for(h, g)), kBlock, 0, h->stream>>>(g, x, h->fluid, h->red, h->s, kz_for(h, g));
   CKL();
   if (!is_pure(h->opts)) {
     // no null space: psi is the solution itself
@@ -1717,7 +1735,7 @@ smac_status smac_time_kernel(smac_handle* h, int kernel_id, int reps, float* ms,
   if (!h || !ms || !bytes || reps < 1) { set_err("smac_time_kernel: bad argument"); return SMAC_BAD_ARG; }
   if (!h->have_coeffs) { set_err("smac_time_kernel: coefficients required"); return SMAC_BAD_ARG; }
   const Geom& g = h->lv[0].g;
-  const int kz = kz_for(g);
+  const int kz = kz_for(h, g);
   // a state in which no kernel early-exits and the updates are no-ops
   Scalars st{};
   st.max_iter = 1 << 30;
@@ -1785,13 +1803,13 @@ smac_status smac_time_kernel(smac_handle* h, int kernel_id, int reps, float* ms,
       }
       case 7: {
         auto S = stencil<float, float>(g, h->lv[0].bxm, h->lv[0].bym, h->lv[0].bzm);
-        launch_dir_matvec<float>(h, g, h->z32, h->d32, h->d32b, S, h->q32, kz);
+        launch_dir_matvec<float>(h, g, h->z32, h->d32, h->d32b, S, h->q32);
         per = 7 * 4.0;
         break;
       }
       case 8: {
         auto S = stencil<double, double>(g, h->lv[0].bx64, h->lv[0].by64, h->lv[0].bz64);
-        launch_dir_matvec<double>(h, g, h->z64, h->d64, h->d64b, S, h->q64, kz);
+        launch_dir_matvec<double>(h, g, h->z64, h->d64, h->d64b, S, h->q64);
         per = 7 * 8.0;
         break;
       }
@@ -1857,7 +1875,7 @@ template <class T, class C>
 smac_status sweep_selftest(smac_handle* h, int mode, T* x, T* xa, T* xb, T* rhs, const void* bx, const void* by,
                            const void* bz, const T* xc, long long* mismatches) {
   const Geom& g = h->lv[0].g;
-  const int kz = kz_for(g);
+  const int kz = kz_for(h, g);
   const Level& Lc = h->lv[1];
   const int c0 = (mode == 2) ? 1 : 0;
   // reference: two in-place half-sweeps on a copy of x
