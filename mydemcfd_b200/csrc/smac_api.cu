@@ -1179,9 +1179,8 @@ smac_status smac_create(const smac_grid_desc* desc, const smac_options* opts, vo
   {
     long long maxb = 0;
     for (int l = 0; l < h->nlev; ++l) {
-      const dim3 gr = grid_cells(h->lv[l].g, kz_for(h, h->lv[l].g));
-      maxb = std::max(maxb, (long long)gr.x * gr.y * gr.z);
-      const dim3 gp = grid_planes(h->lv[l].g.nx, h->lv[l].g.ny, h->lv[l].g.nz);
+      const Geom& g = h->lv[l].g;
+      const dim3 gp = grid_planes(g.nx + 1, g.ny + 1, g.nz + 1);  // one plane per block, faces included: the most
       maxb = std::max(maxb, (long long)gp.x * gp.y * gp.z);
     }
     if ((st = dalloc(h, &h->red.partials, maxb * 4 + 64))) return fail(st);
@@ -1260,42 +1259,27 @@ smac_status smac_set_coefficients(smac_handle* h, const double* fbx, const doubl
     CK(cudaMemcpyAsync(h->fyt, fyt, nyf, cudaMemcpyDeviceToDevice, h->stream));
     CK(cudaMemcpyAsync(h->fzt, fzt, nzf, cudaMemcpyDeviceToDevice, h->stream));
   }
-  k_import_coeffs<<<grid_planes(g.nx + 1, g.ny + 1, g.nz + 1), kBlock, 0, h->stream>>>(
-      g, h->R, fbx, fby, fbz, ct, fxt, fyt, fzt, h->fbx, h->fby, h->fbz, h->lv[0].bx64, h->lv[0].by64,
-      h->lv[0].bz64, h->fluid);
-  CKL();
-  k_fluid_finalize<<<grid_cells(g, kz_for(h, g)), kBlock, 0, h->stream>>>(g, h->fbx, h->fby, h->fbz, h->fluid, h->red,
-                                                                       h->s, kz_for(h, g));
-  CKL();
-  // FP32 fine copy for the mixed-precision Krylov operator
   {
-    const long long n = g.alloc;
-    k_convert<float><<<1184, 256, 0, h->stream>>>(base_of(g, h->lv[0].bx64), base_of(g, (float*)h->lv[0].bxm), n);
-    k_convert<float><<<1184, 256, 0, h->stream>>>(base_of(g, h->lv[0].by64), base_of(g, (float*)h->lv[0].bym), n);
-    k_convert<float><<<1184, 256, 0, h->stream>>>(base_of(g, h->lv[0].bz64), base_of(g, (float*)h->lv[0].bzm), n);
+    const int kz = kz_for(h, g);
+    const dim3 gr((g.nx + 1 + TBX - 1) / TBX, (g.ny + 1 + TBY - 1) / TBY, (g.nz + 1 + kz - 1) / kz);
+    Level& L = h->lv[0];
+    k_import_coeffs<<<gr, kBlock, 0, h->stream>>>(g, h->R, fbx, fby, fbz, ct, fxt, fyt, fzt, h->fbx, h->fby, h->fbz,
+                                                  L.bx64, L.by64, L.bz64, (float*)L.bxm, (float*)L.bym, (float*)L.bzm,
+                                                  h->fluid, h->red, h->s, kz);
     CKL();
   }
   for (int l = 1; l < h->nlev; ++l) {
     Level& F = h->lv[l - 1];
     Level& L = h->lv[l];
     const dim3 gr = grid_planes(L.g.nx + 1, L.g.ny + 1, L.g.nz + 1);
-    k_coarsen_coeffs<double><<<gr, kBlock, 0, h->stream>>>(F.g, L.g, L.cx, L.cy, L.cz, L.ax, L.ay, L.az, F.bx64,
-                                                           F.by64, F.bz64, L.bx64, L.by64, L.bz64, nullptr, nullptr,
-                                                           nullptr);
-    CKL();
-    const long long n = L.g.alloc;
-    if (L.ctm == CT_BF16) {
-      k_convert<__nv_bfloat16><<<256, 256, 0, h->stream>>>(base_of(L.g, L.bx64), base_of(L.g, (__nv_bfloat16*)L.bxm), n);
-      k_convert<__nv_bfloat16><<<256, 256, 0, h->stream>>>(base_of(L.g, L.by64), base_of(L.g, (__nv_bfloat16*)L.bym), n);
-      k_convert<__nv_bfloat16><<<256, 256, 0, h->stream>>>(base_of(L.g, L.bz64), base_of(L.g, (__nv_bfloat16*)L.bzm), n);
-      k_widen_bf16<<<256, 256, 0, h->stream>>>(base_of(L.g, (const __nv_bfloat16*)L.bxm), base_of(L.g, L.bxw), n);
-      k_widen_bf16<<<256, 256, 0, h->stream>>>(base_of(L.g, (const __nv_bfloat16*)L.bym), base_of(L.g, L.byw), n);
-      k_widen_bf16<<<256, 256, 0, h->stream>>>(base_of(L.g, (const __nv_bfloat16*)L.bzm), base_of(L.g, L.bzw), n);
-    } else {
-      k_convert<float><<<256, 256, 0, h->stream>>>(base_of(L.g, L.bx64), base_of(L.g, (float*)L.bxm), n);
-      k_convert<float><<<256, 256, 0, h->stream>>>(base_of(L.g, L.by64), base_of(L.g, (float*)L.bym), n);
-      k_convert<float><<<256, 256, 0, h->stream>>>(base_of(L.g, L.bz64), base_of(L.g, (float*)L.bzm), n);
-    }
+    if (L.ctm == CT_BF16)
+      k_coarsen_coeffs<<<gr, kBlock, 0, h->stream>>>(
+          F.g, L.g, L.cx, L.cy, L.cz, L.ax, L.ay, L.az, F.bx64, F.by64, F.bz64, L.bx64, L.by64, L.bz64,
+          (__nv_bfloat16*)L.bxm, (__nv_bfloat16*)L.bym, (__nv_bfloat16*)L.bzm, L.bxw, L.byw, L.bzw);
+    else
+      k_coarsen_coeffs<<<gr, kBlock, 0, h->stream>>>(
+          F.g, L.g, L.cx, L.cy, L.cz, L.ax, L.ay, L.az, F.bx64, F.by64, F.bz64, L.bx64, L.by64, L.bz64, (float*)L.bxm,
+          (float*)L.bym, (float*)L.bzm, nullptr, nullptr, nullptr);
     CKL();
   }
   TRY(scalars_to_host(h));

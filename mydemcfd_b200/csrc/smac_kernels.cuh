@@ -12,6 +12,8 @@
 // each result rounds exactly like the reference built with -fmad=false.
 #pragma once
 
+#include <type_traits>
+
 #include "smac_common.cuh"
 
 namespace smac {
@@ -34,67 +36,92 @@ constexpr int TNT = TBX * TBY;
 // diagonal, as the reference's Adiag does (G_PCGSolver.cu:168-175).
 // Writes the masked f_b (b*) and the stencil weights w = f_b / h^2 (w*),
 // rounded as the reference's Axp = f_bx * inv_dx2 (G_PCGSolver.cu:168-173).
-__global__ void k_import_coeffs(Geom g, RefDims R, const double* __restrict__ fbx, const double* __restrict__ fby,
-                                const double* __restrict__ fbz, const uint8_t* __restrict__ ct,
-                                const uint8_t* __restrict__ fxt, const uint8_t* __restrict__ fyt,
-                                const uint8_t* __restrict__ fzt, double* bx, double* by, double* bz,
-                                double* wx, double* wy, double* wz, uint8_t* fluid) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  if (i > g.nx || j > g.ny || k > g.nz) return;
-  const int c = g.idx(i, j, k);
-  auto interior_cell = [&](int ii, int jj, int kk) -> int {  // 1 C_INTERIOR, 0 other, -1 outside
-    if (ii < 0 || jj < 0 || kk < 0 || ii >= g.nx || jj >= g.ny || kk >= g.nz) return -1;
-    return ct[R.cell(ii + 1, jj + 1, kk + 1)] == C_INTERIOR ? 1 : 0;
-  };
-  // x-face i between cells i-1 and i
-  if (i <= g.nx && j < g.ny && k < g.nz) {
-    const int a = interior_cell(i - 1, j, k), b = interior_cell(i, j, k);
-    double v = fbx[R.xf(i + 1, j + 1, k + 1)];
-    if (a == 0 || b == 0) v = 0.0;
-    if (a == 1 && b == 1 && fxt[R.xf(i + 1, j + 1, k + 1)] != F_INTERIOR) v = 0.0;
-    bx[c] = v;
-    wx[c] = __dmul_rn(v, g.ihx2);
-  }
-  if (i < g.nx && j <= g.ny && k < g.nz) {
-    const int a = interior_cell(i, j - 1, k), b = interior_cell(i, j, k);
-    double v = fby[R.yf(i + 1, j + 1, k + 1)];
-    if (a == 0 || b == 0) v = 0.0;
-    if (a == 1 && b == 1 && fyt[R.yf(i + 1, j + 1, k + 1)] != F_INTERIOR) v = 0.0;
-    by[c] = v;
-    wy[c] = __dmul_rn(v, g.ihy2);
-  }
-  if (i < g.nx && j < g.ny && k <= g.nz) {
-    const int a = interior_cell(i, j, k - 1), b = interior_cell(i, j, k);
-    double v = fbz[R.zf(i + 1, j + 1, k + 1)];
-    if (a == 0 || b == 0) v = 0.0;
-    if (a == 1 && b == 1 && fzt[R.zf(i + 1, j + 1, k + 1)] != F_INTERIOR) v = 0.0;
-    bz[c] = v;
-    wz[c] = __dmul_rn(v, g.ihz2);
-  }
-  if (i < g.nx && j < g.ny && k < g.nz) fluid[c] = (interior_cell(i, j, k) == 1) ? 1 : 0;
-}
-
-// Cell bits: bit 0 C_INTERIOR, bit 1 fluid (C_INTERIOR with a non-zero
-// diagonal: the cells that carry unknowns).  Counts the fluid cells.
-
-__global__ void __launch_bounds__(TNT) k_fluid_finalize(Geom g, const double* __restrict__ bx,
-                                                        const double* __restrict__ by, const double* __restrict__ bz,
-                                                        uint8_t* fluid, RedBuf red, Scalars* s, int kz) {
+// Also the FP32 weights of the mixed form (m*), the cell bits (bit 0
+// C_INTERIOR, bit 1 fluid: C_INTERIOR with a non-zero diagonal, the cells that
+// carry unknowns) and the number of fluid cells.  One pass: a thread holds the
+// six masked f_b of its cell and marches in z.  (Import, count and FP32
+// conversions used to be five launches here, and four to seven per coarse
+// grid: smac_set_coefficients took 145, 173, 269, 432 and 765 us at 32^3,
+// 64^3, 128^3, 192^3 and 256^3; 66, 73, 158, 310 and 574 now.)
+__global__ void __launch_bounds__(TNT) k_import_coeffs(
+    Geom g, RefDims R, const double* __restrict__ fbx, const double* __restrict__ fby, const double* __restrict__ fbz,
+    const uint8_t* __restrict__ ct, const uint8_t* __restrict__ fxt, const uint8_t* __restrict__ fyt,
+    const uint8_t* __restrict__ fzt, double* __restrict__ bx, double* __restrict__ by, double* __restrict__ bz,
+    double* __restrict__ wx, double* __restrict__ wy, double* __restrict__ wz, float* __restrict__ mx,
+    float* __restrict__ my, float* __restrict__ mz, uint8_t* __restrict__ fluid, RedBuf red, Scalars* s, int kz) {
   const int i = blockIdx.x * TBX + threadIdx.x;
   const int j = blockIdx.y * TBY + threadIdx.y;
   const int k0 = blockIdx.z * kz;
+  // 1 C_INTERIOR, 0 other, -1 outside
+  auto cell = [&](int ii, int jj, int kk) -> int {
+    if (ii < 0 || jj < 0 || kk < 0 || ii >= g.nx || jj >= g.ny || kk >= g.nz) return -1;
+    return ct[R.cell(ii + 1, jj + 1, kk + 1)] == C_INTERIOR ? 1 : 0;
+  };
+  auto masked = [](int a, int b, double v, uint8_t t) -> double {
+    return (a == 0 || b == 0 || (a == 1 && b == 1 && t != F_INTERIOR)) ? 0.0 : v;
+  };
   double v[1] = {0.0};
-  if (i < g.nx && j < g.ny) {
-    const int k1 = min(k0 + kz, g.nz);
+  // The march carries the cell and the z-face of the plane above; the x
+  // neighbours' cells and high faces come from the next lanes (j is uniform in
+  // a warp, lanes past the row take part with nothing to write).
+  if (j <= g.ny) {
+    const int lane = threadIdx.x;
+    const bool xi = i < g.nx, xf = i <= g.nx, yi = j < g.ny;
+    const int k1 = min(k0 + kz, g.nz + 1);
+    int cc = cell(i, j, k0);
+    double zl = 0.0;
+    if (xi && yi) {
+      const long long f = R.zf(i + 1, j + 1, k0 + 1);
+      zl = masked(cell(i, j, k0 - 1), cc, fbz[f], fzt[f]);
+    }
     for (int k = k0; k < k1; ++k) {
       const int c = g.idx(i, j, k);
-      const double d = bx[c] + bx[c + 1] + by[c] + by[c + g.px] + bz[c] + bz[c + g.ps];
-      const uint8_t in = fluid[c] & 1;
-      const uint8_t f = (in && d > 0.0) ? 1 : 0;
-      fluid[c] = (uint8_t)(in | (f << 1));
-      v[0] += f;
+      const bool zi = k < g.nz, in = xi && yi && zi;
+      const int cn = cell(i, j, k + 1), cym = cell(i, j - 1, k), cyp = cell(i, j + 1, k);
+      double fx = 0.0, fxn = 0.0, yl = 0.0, yh = 0.0, zh = 0.0;
+      uint8_t tx = 0, txn = 0;
+      const long long f = R.xf(i + 1, j + 1, k + 1), y = R.yf(i + 1, j + 1, k + 1), z = R.zf(i + 1, j + 1, k + 2);
+      if (xf && yi && zi) {
+        fx = fbx[f];
+        tx = fxt[f];
+        if (lane == 31 && xi) { fxn = fbx[f + 1]; txn = fxt[f + 1]; }
+      }
+      if (xi && zi) {
+        yl = masked(cym, cc, fby[y], fyt[y]);
+        if (yi) yh = masked(cc, cyp, fby[y + R.Nx + 2], fyt[y + R.Nx + 2]);
+      }
+      if (in) zh = masked(cc, cn, fbz[z], fzt[z]);
+      int cxm = __shfl_up_sync(0xffffffffu, cc, 1), cxp = __shfl_down_sync(0xffffffffu, cc, 1);
+      if (lane == 0) cxm = cell(i - 1, j, k);
+      if (lane == 31) cxp = cell(i + 1, j, k);
+      const double xl = masked(cxm, cc, fx, tx);
+      double xh = __shfl_down_sync(0xffffffffu, xl, 1);
+      if (lane == 31) xh = masked(cc, cxp, fxn, txn);
+      if (xf && yi && zi) {
+        const double w = __dmul_rn(xl, g.ihx2);
+        bx[c] = xl;
+        wx[c] = w;
+        mx[c] = (float)w;
+      }
+      if (xi && zi) {
+        const double w = __dmul_rn(yl, g.ihy2);
+        by[c] = yl;
+        wy[c] = w;
+        my[c] = (float)w;
+      }
+      if (xi && yi) {
+        const double w = __dmul_rn(zl, g.ihz2);
+        bz[c] = zl;
+        wz[c] = w;
+        mz[c] = (float)w;
+      }
+      if (in) {
+        const uint8_t u = (cc == 1 && xl + xh + yl + yh + zl + zh > 0.0) ? 1 : 0;
+        fluid[c] = (uint8_t)((cc == 1 ? 1 : 0) | (u << 1));
+        v[0] += u;
+      }
+      cc = cn;
+      zl = zh;
     }
   }
   const Op ops[1] = {Op::Sum};
@@ -132,11 +159,15 @@ inline CoarseAxis coarse_axis(bool halved, int n_fine, double l, double* L) {
 __device__ __forceinline__ double coarse_factor(const CoarseAxis& a, int I, int nc) {
   return I < nc - 1 ? a.regular : I == nc - 1 ? a.last : a.wall;
 }
+// Written as FP64, as C (the mixed form's storage) and, where C is BF16,
+// widened to FP32 for the cluster kernel: one launch per grid.
 template <class C>
 __global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, CoarseAxis ax, CoarseAxis ay, CoarseAxis az,
                                  const double* __restrict__ fbx, const double* __restrict__ fby,
-                                 const double* __restrict__ fbz, C* bx, C* by, C* bz, double* bx64, double* by64,
-                                 double* bz64) {
+                                 const double* __restrict__ fbz, double* __restrict__ bx64, double* __restrict__ by64,
+                                 double* __restrict__ bz64, C* __restrict__ bx, C* __restrict__ by,
+                                 C* __restrict__ bz, float* __restrict__ bxw, float* __restrict__ byw,
+                                 float* __restrict__ bzw) {
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = blockIdx.y * blockDim.y + threadIdx.y;
   const int K = blockIdx.z;
@@ -150,8 +181,9 @@ __global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, Coars
       for (int dj = 0; dj < ry; ++dj)
         if (j0 + dj < gf.ny && k0 + dk < gf.nz) s += fbx[gf.idx(i, j0 + dj, k0 + dk)];
     s *= coarse_factor(ax, I, gc.nx) / (double)(ry * rz);
+    bx64[c] = s;
     bx[c] = coef_from_double<C>(s);
-    if (bx64) bx64[c] = s;
+    if constexpr (std::is_same<C, __nv_bfloat16>::value) bxw[c] = __bfloat162float(bx[c]);
   }
   if (I < gc.nx && K < gc.nz) {  // y-face J
     const int jj = cy ? min(2 * J, gf.ny) : J, i0 = cx ? 2 * I : I, k0 = cz ? 2 * K : K;
@@ -160,8 +192,9 @@ __global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, Coars
       for (int di = 0; di < rx; ++di)
         if (i0 + di < gf.nx && k0 + dk < gf.nz) s += fby[gf.idx(i0 + di, jj, k0 + dk)];
     s *= coarse_factor(ay, J, gc.ny) / (double)(rx * rz);
+    by64[c] = s;
     by[c] = coef_from_double<C>(s);
-    if (by64) by64[c] = s;
+    if constexpr (std::is_same<C, __nv_bfloat16>::value) byw[c] = __bfloat162float(by[c]);
   }
   if (I < gc.nx && J < gc.ny) {  // z-face K
     const int kk = cz ? min(2 * K, gf.nz) : K, i0 = cx ? 2 * I : I, j0 = cy ? 2 * J : J;
@@ -170,8 +203,9 @@ __global__ void k_coarsen_coeffs(Geom gf, Geom gc, int cx, int cy, int cz, Coars
       for (int di = 0; di < rx; ++di)
         if (i0 + di < gf.nx && j0 + dj < gf.ny) s += fbz[gf.idx(i0 + di, j0 + dj, kk)];
     s *= coarse_factor(az, K, gc.nz) / (double)(rx * ry);
+    bz64[c] = s;
     bz[c] = coef_from_double<C>(s);
-    if (bz64) bz64[c] = s;
+    if constexpr (std::is_same<C, __nv_bfloat16>::value) bzw[c] = __bfloat162float(bz[c]);
   }
 }
 
@@ -186,18 +220,11 @@ __global__ void k_zero16(int4* p, long long n16) {
     p[t] = make_int4(0, 0, 0, 0);
 }
 
-// FP64 -> C copy of a whole padded array (fine-level FP32 / BF16 coefficients).
+// FP64 -> C copy of a whole padded array (the kernel timings' operands).
 template <class C>
 __global__ void k_convert(const double* __restrict__ a, C* b, long long n) {
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   for (; t < n; t += (long long)gridDim.x * blockDim.x) b[t] = coef_from_double<C>(a[t]);
-}
-
-// BF16 -> FP32 copy of a whole padded array (exact): the cluster kernel's
-// copy of the BF16 coefficients, which it stages without conversion.
-__global__ void k_widen_bf16(const __nv_bfloat16* __restrict__ a, float* b, long long n) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  for (; t < n; t += (long long)gridDim.x * blockDim.x) b[t] = __bfloat162float(a[t]);
 }
 
 // ------------------------------------------------------------------------
