@@ -129,7 +129,7 @@ struct smac_handle {
   struct ClusterPlan {
     int lk = -1, nd = 0;
     int chunk[MAXL] = {}, off[MAXL][5] = {};
-    int elems = 0;
+    int elems = 0, scratch = -1;
   } kc[2];
   Level lv[MAXL];
   uint8_t* fluid = nullptr;   // padded cell bits: 1 C_INTERIOR, 2 fluid unknown
@@ -541,6 +541,7 @@ void launch_cluster(smac_handle* h, bool mixed, const T* rhs, T* x) {
   ClusterSet set{};
   set.n = h->nlev - P.lk;
   set.nd = P.nd;
+  set.scratch = P.scratch;
   for (int q = 0; q < set.n; ++q) {
     const Level& L = h->lv[P.lk + q];
     ClusterLevel& C = set.L[q];
@@ -551,7 +552,6 @@ void launch_cluster(smac_handle* h, bool mixed, const T* rhs, T* x) {
     C.obx = P.off[q][2]; C.oby = P.off[q][3]; C.obz = P.off[q][4];
     // every array staged as T: BF16 weights through their exact FP32 copies
     const bool wide = mixed && L.ctm == CT_BF16;
-    C.ctype = mixed ? CT_F32 : CT_F64;
     C.bx = wide ? (const void*)L.bxw : mixed ? L.bxm : (const void*)L.bx64;
     C.by = wide ? (const void*)L.byw : mixed ? L.bym : (const void*)L.by64;
     C.bz = wide ? (const void*)L.bzw : mixed ? L.bzm : (const void*)L.bz64;
@@ -939,7 +939,7 @@ bool plan_cluster(smac_handle* h, int lk, int smem_optin) {
   const int nz0 = h->lv[lk].g.nz;
   int chunk = (nz0 + KCL - 1) / KCL;
   chunk = (chunk + pow2 - 1) / pow2 * pow2;
-  long long tot = 0;
+  long long tot = 0, cells = 0;
   auto take = [&](long long e) { const long long o = tot; tot += (e + 3) / 4 * 4; return (int)o; };
   for (int q = 0; q < n; ++q) {
     const Geom& g = h->lv[lk + q].g;
@@ -948,6 +948,7 @@ bool plan_cluster(smac_handle* h, int lk, int smem_optin) {
     if (c < 1) return false;
     P.chunk[q] = c;
     const long long nx = g.nx, ny = g.ny;
+    cells = std::max(cells, c * nx * ny);
     P.off[q][0] = take(c * nx * ny);            // x
     P.off[q][1] = take(c * nx * ny);            // rhs
     P.off[q][2] = take(c * ny * (nx + 1));      // bx
@@ -955,6 +956,8 @@ bool plan_cluster(smac_handle* h, int lk, int smem_optin) {
     P.off[q][4] = take((c + 1) * ny * nx);      // bz
     if (tot * (int)sizeof(T) > smem_optin) return false;
   }
+  // (FP64 at 32^3 leaves no room for the residuals)
+  P.scratch = (tot + cells + 3) * (int)sizeof(T) <= smem_optin ? take(cells) : -1;
   if (!cluster_attr<T>((int)(tot * (int)sizeof(T)))) return false;
   P.elems = (int)tot;
   P.nd = nd;

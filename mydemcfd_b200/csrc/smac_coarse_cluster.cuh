@@ -54,14 +54,14 @@ struct ClusterLevel {
   int cx, cy, cz;     // how this grid was coarsened from the one above
   int chunk;          // planes per rank (nz for a grid held by rank 0)
   int ox, orhs, obx, oby, obz;
-  int ctype;          // global coefficient storage: 0 FP64, 1 FP32, 2 BF16
-  const void* bx;
+  const void* bx;     // weights, stored as T
   const void* by;
   const void* bz;
 };
 struct ClusterSet {
   ClusterLevel L[MAX_CLL];
   int n;        // grids in the set
+  int scratch;  // offset of the residuals of a chunk of cells (-1: no room)
   int nd;       // the first nd are spread over the ranks, the rest held by rank 0
   const void* rhs0;  // right-hand side of L[0] (global, padded layout)
   void* x0;          // its result (global, padded layout; the pads are not written)
@@ -100,54 +100,43 @@ struct ClusterView {
   }
 };
 
-// Copies nrows rows of rl elements (global row r at src + base + (r / rpp) *
-// ps + (r % rpp) * px, for rpp rows per plane) into dst, row after row.  The
-// warps take rows in turn and the lanes a row's elements: one division per
-// row.  Arrays stored as T are copied by asynchronous element copies (all of
-// a thread's copies in flight; the caller waits), others through registers
-// (converted exactly to T).
+// Copies planes of rows of rl elements (global row j of plane k at src + base +
+// k ps + j px, rpp rows per plane) into dst, row after row.  The warps take a
+// plane's rows in turn and the lanes a row's elements, by asynchronous element
+// copies (all of a thread's copies in flight; the caller waits).
 template <class T>
-__device__ __forceinline__ void cl_copy_rows(T* dst, const void* src, int ctype, int base, int nrows, int rl,
-                                             int rpp, int px, int ps) {
+__device__ __forceinline__ void cl_copy_rows(T* dst, const T* src, int base, int planes, int rl, int rpp, int px,
+                                             int ps) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const bool same = ctype == (sizeof(T) == 8 ? 0 : 1);
-  for (int r = w; r < nrows; r += nw) {
-    const int g0 = base + (r / rpp) * ps + (r % rpp) * px;
-    T* d = dst + r * rl;
-    if (same) {
-      const T* sp = reinterpret_cast<const T*>(src) + g0;
-      for (int i = lane; i < rl; i += 32) __pipeline_memcpy_async(d + i, sp + i, sizeof(T));
-    } else {
-      for (int i = lane; i < rl; i += 32) {
-        if (ctype == 0) d[i] = (T)reinterpret_cast<const double*>(src)[g0 + i];
-        else if (ctype == 1) d[i] = (T)reinterpret_cast<const float*>(src)[g0 + i];
-        else d[i] = (T)__bfloat162float(reinterpret_cast<const __nv_bfloat16*>(src)[g0 + i]);
-      }
-    }
+  for (int k = 0; k < planes; ++k) {
+    const T* sp = src + base + k * ps;
+    T* d = dst + k * rpp * rl;
+#pragma unroll 2
+    for (int j = w; j < rpp; j += nw)
+      for (int i = lane; i < rl; i += 32) __pipeline_memcpy_async(d + j * rl + i, sp + j * px + i, sizeof(T));
   }
 }
 
-// The weights of this rank's planes of grid L and, for the set's first grid,
-// its right-hand side, into shared memory.
+// The weights of this rank's planes of grid L, or its right-hand side, into
+// shared memory.
 template <class T>
-__device__ __noinline__ void cl_stage(ClusterView<T> V, const ClusterLevel& Lp, const T* rhs0) {
+__device__ __noinline__ void cl_stage(ClusterView<T> V, const ClusterLevel& Lp) {
   const ClGrid L = cl_grid(Lp);
   const Geom& g = Lp.g;
   const int k0 = V.p0(L), np = V.p1(L) - k0;
   if (np <= 0) return;
   const int b = g.idx(0, 0, k0);
-  cl_copy_rows<T>(V.local + L.obx, Lp.bx, Lp.ctype, b, np * L.ny, L.nx + 1, L.ny, g.px, g.ps);
-  cl_copy_rows<T>(V.local + L.oby, Lp.by, Lp.ctype, b, np * (L.ny + 1), L.nx, L.ny + 1, g.px, g.ps);
-  cl_copy_rows<T>(V.local + L.obz, Lp.bz, Lp.ctype, b, (np + 1) * L.ny, L.nx, L.ny, g.px, g.ps);  // z-faces k0..k0+np
-  if (rhs0) cl_copy_rows<T>(V.local + L.orhs, rhs0, sizeof(T) == 8 ? 0 : 1, b, np * L.ny, L.nx, L.ny, g.px, g.ps);
+  cl_copy_rows<T>(V.local + L.obx, (const T*)Lp.bx, b, np, L.nx + 1, L.ny, g.px, g.ps);
+  cl_copy_rows<T>(V.local + L.oby, (const T*)Lp.by, b, np, L.nx, L.ny + 1, g.px, g.ps);
+  cl_copy_rows<T>(V.local + L.obz, (const T*)Lp.bz, b, np + 1, L.nx, L.ny, g.px, g.ps);  // z-faces k0..k0+np
 }
 template <class T>
-__device__ __noinline__ void cl_stage_rhs(ClusterView<T> V, const ClusterLevel& Lp, const T* rhs0) {
+__device__ __forceinline__ void cl_stage_rhs(ClusterView<T> V, const ClusterLevel& Lp, const T* rhs0) {
   const ClGrid L = cl_grid(Lp);
   const Geom& g = Lp.g;
   const int k0 = V.p0(L), np = V.p1(L) - k0;
   if (np <= 0) return;
-  cl_copy_rows<T>(V.local + L.orhs, rhs0, sizeof(T) == 8 ? 0 : 1, g.idx(0, 0, k0), np * L.ny, L.nx, L.ny, g.px, g.ps);
+  cl_copy_rows<T>(V.local + L.orhs, rhs0, g.idx(0, 0, k0), np, L.nx, L.ny, g.px, g.ps);
 }
 
 // The six neighbours (x-, x+, y-, y+, z-, z+) of the own cell (i, j, k) of
@@ -186,57 +175,66 @@ __device__ __forceinline__ void cl_weights(const ClusterView<T>& V, const ClGrid
   wzp = bz[nx * ny];
 }
 
-// Half-sweep of colour `colour` over this rank's planes of grid L: the
-// operations of cta_half_sweep.  pro: with the prolongation of the coarse
-// grid Lc's x added to every neighbour inside the grid.  A thread's items are
-// t, t + blockDim, ... of the (pair, row, plane) box; their coordinates
-// advance by carries, with no division inside the loop.
+// A thread's items t, t + blockDim, ... of the (pair, row, plane) box of this
+// rank's planes: the first one's coordinates and the steps to the next, found
+// once per grid (they take six integer divisions).
+struct ClItems {
+  int total, tx, j, kk, sx, sj, sk;
+};
 template <class T>
-__device__ __noinline__ void cl_half_sweep(ClusterView<T> V, ClGrid L, int colour, bool zero_init, bool pro,
-                                           ClGrid Lc) {
+__device__ __forceinline__ ClItems cl_items(const ClusterView<T>& V, const ClGrid& L) {
+  const int half = (L.nx + 1) / 2, t = threadIdx.x, s = blockDim.x;
+  return ClItems{half * L.ny * max(0, V.p1(L) - V.p0(L)), t % half, (t / half) % L.ny, t / (half * L.ny),
+                 s % half, (s / half) % L.ny, s / (half * L.ny)};
+}
+
+// Half-sweep of colour `colour` over this rank's planes of grid L: the
+// operations of cta_half_sweep.  The items' coordinates advance by carries.
+template <class T>
+__device__ __noinline__ void cl_half_sweep(ClusterView<T> V, ClGrid L, ClItems I, int colour, bool zero_init) {
   typedef acc_t<T> A;
   const int nx = L.nx, ny = L.ny, k0 = V.p0(L), np = V.p1(L) - k0;
   const int half = (nx + 1) / 2;
-  const int total = half * ny * max(0, np);
-  int t = threadIdx.x;
-  if (t >= total) return;
-  int tx = t % half, j = (t / half) % ny, kk = t / (half * ny);
-  const int st = blockDim.x, sx = st % half, sj = (st / half) % ny, sk = st / (half * ny);
-  for (; t < total; t += st) {
+  int tx = I.tx, j = I.j, kk = I.kk;
+  for (int t = threadIdx.x; t < I.total; t += blockDim.x) {
     const int k = k0 + kk;
     const int i = 2 * tx + ((2 * tx + j + k + colour) & 1);
     if (i < nx) {
       const int c = (kk * ny + j) * nx + i;
-      T wxm, wxp, wym, wyp, wzm, wzp;
+      T wxm, wxp, wym, wyp, wzm, wzp, n[6] = {(T)0, (T)0, (T)0, (T)0, (T)0, (T)0};
       cl_weights(V, L, i, j, kk, c, wxm, wxp, wym, wyp, wzm, wzp);
       const A bv = (A)V.local[L.orhs + c];  // (no mean shift below the finest grid)
-      A n[6] = {(A)0, (A)0, (A)0, (A)0, (A)0, (A)0};
-      if (!zero_init) {
-        T xn[6];
-        cl_nb(V, L, i, j, k, kk, np, c, xn);
-#pragma unroll
-        for (int q = 0; q < 6; ++q) n[q] = (A)xn[q];
-        if (pro) {
-          const int ci[6][3] = {{i - 1, j, k}, {i + 1, j, k}, {i, j - 1, k}, {i, j + 1, k}, {i, j, k - 1},
-                                {i, j, k + 1}};
-#pragma unroll
-          for (int q = 0; q < 6; ++q) {
-            const int a = ci[q][0], b = ci[q][1], d = ci[q][2];
-            if (a >= 0 && b >= 0 && d >= 0 && a < nx && b < ny && d < L.nz)
-              n[q] = Ar<A>::add(n[q], (A)V.x(Lc, Lc.cx ? a >> 1 : a, Lc.cy ? b >> 1 : b, Lc.cz ? d >> 1 : d));
-          }
-        }
-      }
-      V.local[L.ox + c] = (T)Stencil<T, T>::gs(bv, (A)wxm, (A)wxp, (A)wym, (A)wyp, (A)wzm, (A)wzp, n[0], n[1], n[2],
-                                               n[3], n[4], n[5]);
+      if (!zero_init) cl_nb(V, L, i, j, k, kk, np, c, n);
+      V.local[L.ox + c] = (T)Stencil<T, T>::gs(bv, (A)wxm, (A)wxp, (A)wym, (A)wyp, (A)wzm, (A)wzp, (A)n[0], (A)n[1],
+                                               (A)n[2], (A)n[3], (A)n[4], (A)n[5]);
     }
-    tx += sx;
+    tx += I.sx;
     int cy = tx >= half;
     tx -= cy ? half : 0;
-    j += sj + cy;
+    j += I.sj + cy;
     cy = j >= ny;
     j -= cy ? ny : 0;
-    kk += sk + cy;
+    kk += I.sk + cy;
+  }
+}
+
+// x += P xc on every own cell: the prolongation of Lc's x, ahead of the first
+// post-smoothing sweep (whose first half-sweep reads the sum at the
+// neighbours, and overwrites the rest).  A coarse plane of a spread grid is in
+// the rank of its children, a grid of rank 0 is read from there.
+template <class T>
+__device__ __noinline__ void cl_prolong(ClusterView<T> V, ClGrid L, ClGrid Lc, bool lc_spread) {
+  typedef acc_t<T> A;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int k0 = V.p0(L), np = V.p1(L) - k0, K0 = lc_spread ? V.p0(Lc) : 0;
+  const T* xc = V.at(lc_spread ? V.me : 0, Lc.ox);
+  for (int kk = 0; kk < np; ++kk) {
+    const T* pc = xc + ((Lc.cz ? (k0 + kk) >> 1 : k0 + kk) - K0) * Lc.ny * Lc.nx;
+    for (int j = w; j < L.ny; j += nw) {
+      const T* row = pc + (Lc.cy ? j >> 1 : j) * Lc.nx;
+      T* x = V.local + L.ox + (kk * L.ny + j) * L.nx;
+      for (int i = lane; i < L.nx; i += 32) x[i] = (T)Ar<A>::add((A)x[i], (A)row[Lc.cx ? i >> 1 : i]);
+    }
   }
 }
 
@@ -281,69 +279,84 @@ __device__ __noinline__ void cl_resid_restrict(ClusterView<T> V, ClGrid L, ClGri
   }
 }
 
-// nhalf half-sweeps of a grid held whole by rank 0 (nx*ny*nz <= KCL_SOLO <=
-// blockDim.x): thread t keeps cell t's weights and rhs in registers across
-// the half-sweeps, which read the neighbours' x from shared memory and end
-// at a CTA barrier.  Half-sweep h has colour c0 ^ (h & 1) before swap_at and
-// (1 - c0) ^ ((h - swap_at) & 1) from there (the coarsest grid's backward
-// pairs); the first starts from zero (zero_first) or adds the prolongation
-// of Lc's x to the neighbours (pro_first).  The operations are those of
-// cl_half_sweep.  Called by every thread of rank 0.
+// The same in two passes where the shared memory has room for the residuals of
+// a chunk (at `scratch`): every own cell's residual, row by row without bank
+// conflicts, then the children's sums.
 template <class T>
-__device__ __noinline__ void cl_solo_run(ClusterView<T> V, ClGrid L, int nhalf, int c0, int swap_at, bool zero_first,
-                                         bool pro_first, ClGrid Lc) {
+__device__ __noinline__ void cl_resid_restrict2(ClusterView<T> V, ClGrid L, ClGrid Lc, int scratch) {
   typedef acc_t<T> A;
-  const int nx = L.nx, ny = L.ny, nz = L.nz, pc = nx, pl = nx * ny;
-  const int t = threadIdx.x;
-  const bool own = t < nx * ny * nz;
-  int i = 0, j = 0, k = 0, c = 0;
-  T wxm = (T)0, wxp = (T)0, wym = (T)0, wyp = (T)0, wzm = (T)0, wzp = (T)0;
-  A bv = (A)0;
-  if (own) {
-    i = t % nx;
-    j = (t / nx) % ny;
-    k = t / pl;
-    c = (k * ny + j) * pc + i;
-    cl_weights(V, L, i, j, k, c, wxm, wxp, wym, wyp, wzm, wzp);
-    bv = (A)V.local[L.orhs + c];  // (no mean shift below the finest grid)
-  }
-  T* x = V.local + L.ox;
-  for (int h = 0; h < nhalf; ++h) {
-    const int colour = h < swap_at ? (c0 ^ (h & 1)) : ((1 - c0) ^ ((h - swap_at) & 1));
-    if (own && ((i + j + k + colour) & 1) == 0) {
-      A n[6] = {(A)0, (A)0, (A)0, (A)0, (A)0, (A)0};
-      if (!(h == 0 && zero_first)) {
-        n[0] = (A)(i > 0 ? x[c - 1] : (T)0);
-        n[1] = (A)(i + 1 < nx ? x[c + 1] : (T)0);
-        n[2] = (A)(j > 0 ? x[c - pc] : (T)0);
-        n[3] = (A)(j + 1 < ny ? x[c + pc] : (T)0);
-        n[4] = (A)(k > 0 ? x[c - pl] : (T)0);
-        n[5] = (A)(k + 1 < nz ? x[c + pl] : (T)0);
-        if (h == 0 && pro_first) {
-          const int ci[6][3] = {{i - 1, j, k}, {i + 1, j, k}, {i, j - 1, k}, {i, j + 1, k}, {i, j, k - 1},
-                                {i, j, k + 1}};
-#pragma unroll
-          for (int q = 0; q < 6; ++q) {
-            const int a = ci[q][0], b = ci[q][1], d = ci[q][2];
-            if (a >= 0 && b >= 0 && d >= 0 && a < nx && b < ny && d < nz)
-              n[q] = Ar<A>::add(n[q], (A)V.x(Lc, Lc.cx ? a >> 1 : a, Lc.cy ? b >> 1 : b, Lc.cz ? d >> 1 : d));
-          }
-        }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nx = L.nx, ny = L.ny, k0 = V.p0(L), k1 = V.p1(L), np = k1 - k0;
+  T* res = V.local + scratch;
+  for (int kk = 0; kk < np; ++kk)
+    for (int j = w; j < ny; j += nw)
+      for (int i = lane; i < nx; i += 32) {
+        A r = (A)0;
+        cl_resid_add(V, L, i, j, k0 + kk, kk, np, r);
+        res[(kk * ny + j) * nx + i] = (T)r;
       }
-      x[c] = (T)Stencil<T, T>::gs(bv, (A)wxm, (A)wxp, (A)wym, (A)wyp, (A)wzm, (A)wzp, n[0], n[1], n[2], n[3], n[4],
-                                  n[5]);
-    }
-    __syncthreads();
-  }
+  __syncthreads();
+  const int rx = Lc.cx ? 2 : 1, ry = Lc.cy ? 2 : 1, rz = Lc.cz ? 2 : 1;
+  const int K0 = (k0 + rz - 1) / rz, K1 = min(Lc.nz, (k1 + rz - 1) / rz);
+  for (int K = K0; K < K1; ++K)
+    for (int J = w; J < Lc.ny; J += nw)
+      for (int I = lane; I < Lc.nx; I += 32) {
+        A acc = (A)0;
+        for (int dk = 0; dk < rz; ++dk)
+          for (int dj = 0; dj < ry; ++dj)
+            for (int di = 0; di < rx; ++di) {
+              const int i = (Lc.cx ? 2 * I : I) + di, j = (Lc.cy ? 2 * J : J) + dj, k = (Lc.cz ? 2 * K : K) + dk;
+              if (i >= nx || j >= ny || k >= L.nz) continue;  // no such child (odd extent)
+              acc = Ar<A>::add(acc, (A)res[((k - k0) * ny + j) * nx + i]);
+            }
+        *V.rhsp(Lc, I, J, K) = (T)Ar<A>::div(acc, (A)(rx * ry * rz));
+      }
 }
 
-// Smoothing step helpers: the spread grids end each step at a cluster
-// barrier, the grids of rank 0 at a CTA barrier (rank 0 only).
-template <class T, class F>
-__device__ __forceinline__ void cl_step(const ClusterView<T>& V, bool spread, F&& f) {
-  if (spread || V.me == 0) f();
-  if (spread) cooperative_groups::this_cluster().sync();
-  else if (V.me == 0) __syncthreads();
+// nhalf half-sweeps of a grid held whole by rank 0 (nx*ny*nz <= KCL_SOLO <=
+// blockDim.x): thread t keeps cell t's weights, rhs and reciprocal diagonal in
+// registers across the half-sweeps, which read the neighbours' x from shared
+// memory and end at a barrier of the warps that own cells (the others wait at
+// the one after the last).  Half-sweep h has colour c0 ^ (h & 1) before
+// swap_at and (1 - c0) ^ ((h - swap_at) & 1) from there (the coarsest grid's
+// backward pairs); the first may start from zero (zero_first).  The operations
+// are those of cl_half_sweep.  Called by every thread of rank 0.
+template <class T>
+__device__ __noinline__ void cl_solo_run(ClusterView<T> V, ClGrid L, int nhalf, int c0, int swap_at, bool zero_first) {
+  typedef acc_t<T> A;
+  const int nx = L.nx, ny = L.ny, nz = L.nz, pl = nx * ny, cells = pl * nz;
+  const int t = threadIdx.x, nthreads = (cells + 31) & ~31;
+  if (t < nthreads) {
+    const bool own = t < cells;
+    const int c = own ? t : 0;
+    const int k = c / pl, j = (c - k * pl) / nx, i = c - k * pl - j * nx;
+    T wxm, wxp, wym, wyp, wzm, wzp;
+    cl_weights(V, L, i, j, k, c, wxm, wxp, wym, wyp, wzm, wzp);
+    const A bv = (A)V.local[L.orhs + c];  // (no mean shift below the finest grid)
+    const A d = Stencil<T, T>::diag((A)wxm, (A)wxp, (A)wym, (A)wyp, (A)wzm, (A)wzp);
+    const A rd = d > (A)0 ? Ar<A>::rcp(d) : (A)0;
+    T* x = V.local + L.ox + c;
+    for (int h = 0; h < nhalf; ++h) {
+      const int colour = h < swap_at ? (c0 ^ (h & 1)) : ((1 - c0) ^ ((h - swap_at) & 1));
+      if (own && ((i + j + k + colour) & 1) == 0) {
+        A n[6] = {(A)0, (A)0, (A)0, (A)0, (A)0, (A)0};
+        if (!(h == 0 && zero_first)) {
+          if (i > 0) n[0] = (A)x[-1];
+          if (i + 1 < nx) n[1] = (A)x[1];
+          if (j > 0) n[2] = (A)x[-nx];
+          if (j + 1 < ny) n[3] = (A)x[nx];
+          if (k > 0) n[4] = (A)x[-pl];
+          if (k + 1 < nz) n[5] = (A)x[pl];
+        }
+        const A v = Stencil<T, T>::offsum(bv, (A)wxm, (A)wxp, (A)wym, (A)wyp, (A)wzm, (A)wzp, n[0], n[1], n[2], n[3],
+                                          n[4], n[5]);
+        *x = d > (A)0 ? (T)Ar<A>::mul(v, rd) : (T)0;
+      }
+      if (nthreads <= 32) __syncwarp();
+      else asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+    }
+  }
+  __syncthreads();
 }
 
 // The lower part of the V-cycle: pre-smoothing (nu1 sweeps from zero) and
@@ -364,7 +377,7 @@ __global__ void __cluster_dims__(KCL, 1, 1) __launch_bounds__(kcl_threads<T>())
   const int n = set.n, nd = set.nd;
   // The weights, which no kernel of the solve writes, are staged while the
   // previous kernel drains; the first grid's rhs, its output, after the wait.
-  for (int q = 0; q < n; ++q) cl_stage<T>(V, set.L[q], nullptr);
+  for (int q = 0; q < n; ++q) cl_stage<T>(V, set.L[q]);
   pdl_enter();
   if (s && s->done) {  // the same flag for every rank: all return, or none
     __pipeline_commit();
@@ -375,36 +388,50 @@ __global__ void __cluster_dims__(KCL, 1, 1) __launch_bounds__(kcl_threads<T>())
   __pipeline_commit();
   __pipeline_wait_prior(0);
   cl.sync();
+  auto restrict_to = [&](const ClGrid& L, int q) {  // grid q's residual to grid q + 1
+    const ClGrid C = cl_grid(set.L[q + 1]);
+    if (set.scratch >= 0) cl_resid_restrict2<T>(V, L, C, set.scratch);
+    else cl_resid_restrict<T>(V, L, C);
+  };
   // down the spread grids
   for (int q = 0; q < nd; ++q) {
     const ClGrid L = cl_grid(set.L[q]);
-    for (int it = 0; it < nu1; ++it) {
-      cl_step(V, true, [&] { cl_half_sweep<T>(V, L, 0, it == 0, false, L); });
-      cl_step(V, true, [&] { cl_half_sweep<T>(V, L, 1, false, false, L); });
+    const ClItems I = cl_items<T>(V, L);
+    for (int h = 0; h < 2 * nu1; ++h) {
+      cl_half_sweep<T>(V, L, I, h & 1, h == 0);
+      cl.sync();
     }
-    cl_step(V, true, [&] { cl_resid_restrict<T>(V, L, cl_grid(set.L[q + 1])); });
+    restrict_to(L, q);
+    cl.sync();
   }
   // the grids of rank 0: down, the coarsest, up
   if (V.me == 0) {
     for (int q = nd; q < n - 1; ++q) {
       const ClGrid L = cl_grid(set.L[q]);
-      cl_solo_run<T>(V, L, 2 * nu1, 0, 2 * nu1, true, false, L);
-      cl_step(V, false, [&] { cl_resid_restrict<T>(V, L, cl_grid(set.L[q + 1])); });
+      cl_solo_run<T>(V, L, 2 * nu1, 0, 2 * nu1, true);
+      restrict_to(L, q);
+      __syncthreads();
     }
-    const ClGrid C = cl_grid(set.L[n - 1]);
-    cl_solo_run<T>(V, C, 4 * coarse_pairs, 0, 2 * coarse_pairs, true, false, C);
+    cl_solo_run<T>(V, cl_grid(set.L[n - 1]), 4 * coarse_pairs, 0, 2 * coarse_pairs, true);
     for (int q = n - 2; q >= nd; --q) {
       const ClGrid L = cl_grid(set.L[q]);
-      cl_solo_run<T>(V, L, 2 * nu2, 1, 2 * nu2, false, true, cl_grid(set.L[q + 1]));
+      cl_prolong<T>(V, L, cl_grid(set.L[q + 1]), false);
+      __syncthreads();
+      cl_solo_run<T>(V, L, 2 * nu2, 1, 2 * nu2, false);
     }
   }
   cl.sync();
   // up the spread grids
   for (int q = nd - 1; q >= 0; --q) {
     const ClGrid L = cl_grid(set.L[q]);
-    for (int it = 0; it < nu2; ++it) {
-      cl_step(V, true, [&] { cl_half_sweep<T>(V, L, 1, false, it == 0, cl_grid(set.L[q + 1])); });
-      cl_step(V, true, [&] { cl_half_sweep<T>(V, L, 0, false, false, L); });
+    const ClItems I = cl_items<T>(V, L);
+    if (q + 1 < n) {
+      cl_prolong<T>(V, L, cl_grid(set.L[q + 1]), q + 1 < nd);
+      cl.sync();
+    }
+    for (int h = 0; h < 2 * nu2; ++h) {
+      cl_half_sweep<T>(V, L, I, (h & 1) ^ 1, false);
+      cl.sync();
     }
   }
   // the first grid's x back to global memory (own planes; after the last
