@@ -1375,16 +1375,21 @@ smac_status smac_divergence(smac_handle* h, const double* vxs, const double* vys
   if (!((fsx && fsy && fsz) || (!fsx && !fsy && !fsz))) { set_err("smac_divergence: fsx/fsy/fsz go together"); return SMAC_BAD_ARG; }
   if (!(dt > 0) || !std::isfinite(dt)) { set_err("smac_divergence: dt must be > 0"); return SMAC_BAD_ARG; }
   const Geom& g = h->lv[0].g;
-  if (!eps && !fsx) {
-    constexpr int KZ = 4;
-    k_divergence_z<KZ><<<dim3((g.nx + TBX - 1) / TBX, (g.ny + TBY - 1) / TBY, (g.nz + KZ - 1) / KZ), kBlock, 0,
-                         h->stream>>>(g, h->R, 1.0 / h->desc.dx, 1.0 / h->desc.dy, 1.0 / h->desc.dz, 1.0 / dt, vxs,
-                                      vys, vzs, h->fluid, h->b64, rhs_out);
-  } else {
-    k_divergence<<<grid_planes(g.nx, g.ny, g.nz), kBlock, 0, h->stream>>>(
-        g, h->R, 1.0 / h->desc.dx, 1.0 / h->desc.dy, 1.0 / h->desc.dz, 1.0 / dt, vxs, vys, vzs, eps, eps_old,
-        h->fbx, h->fby, h->fbz, fsx, fsy, fsz, h->fluid, h->b64, rhs_out);
-  }
+  auto launch = [&](auto kz, auto e, auto f) {
+    constexpr int KZ = decltype(kz)::value;
+    k_divergence<KZ, decltype(e)::value, decltype(f)::value>
+        <<<dim3((g.nx + TBX - 1) / TBX, (g.ny + TBY - 1) / TBY, (g.nz + KZ - 1) / KZ), kBlock, 0, h->stream>>>(
+            g, h->R, 1.0 / h->desc.dx, 1.0 / h->desc.dy, 1.0 / h->desc.dz, 1.0 / dt, vxs, vys, vzs, eps, eps_old,
+            h->fbx, h->fby, h->fbz, fsx, fsy, fsz, h->fluid, h->b64, rhs_out);
+  };
+  constexpr std::true_type on{};
+  constexpr std::false_type off{};
+  constexpr std::integral_constant<int, 4> four{};
+  constexpr std::integral_constant<int, 2> two{};  // (more loads per plane)
+  if (eps && fsx) launch(two, on, on);
+  else if (eps) launch(two, on, off);
+  else if (fsx) launch(two, off, on);
+  else launch(four, off, off);
   CKL();
   h->dt = dt;
   h->have_rhs = true;
@@ -1630,9 +1635,9 @@ smac_status smac_correct(smac_handle* h, double* p_delta, double* p, const doubl
   if (!((fsx && fsy && fsz) || (!fsx && !fsy && !fsz))) { set_err("smac_correct: fs* go together"); return SMAC_BAD_ARG; }
   const Geom& g = h->lv[0].g;
   const RefDims& R = h->R;
-  k_correct<<<grid_planes(R.Nx + 3, R.Ny + 3, R.Nz + 3), kBlock, 0, h->stream>>>(
+  k_correct<<<grid_planes(R.Nx + 2, R.Ny + 2, R.Nz + 2), kBlock, 0, h->stream>>>(
       R, g, 1.0 / h->desc.dx, 1.0 / h->desc.dy, 1.0 / h->desc.dz, dt, h->ct, h->fxt, h->fyt, h->fzt, p_delta, p, vxs,
-      vys, vzs, firx, firy, firz, h->fbx, h->fby, h->fbz, fsx, fsy, fsz, vx, vy, vz, 0);
+      vys, vzs, firx, firy, firz, h->fbx, h->fby, h->fbz, fsx, fsy, fsz, vx, vy, vz);
   CKL();
   account(h, g, 3 * 8 + 8 + 3 * 8 + 3 * 8 + 3, 1);
   if (zero_p_delta) {

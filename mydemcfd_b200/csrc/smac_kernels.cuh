@@ -235,94 +235,94 @@ __global__ void k_convert(const double* __restrict__ a, C* b, long long n) {
 // cell: the masked faces carry f_b = 0 in the reference as well).
 // `cellbits` bit 0 marks C_INTERIOR cells.  Writes the padded rhs and
 // optionally the reference-layout rhs.
-__global__ void k_divergence(Geom g, RefDims R, double inv_dx, double inv_dy, double inv_dz, double inv_dt,
-                             const double* __restrict__ vx, const double* __restrict__ vy,
-                             const double* __restrict__ vz, const double* __restrict__ eps,
-                             const double* __restrict__ eps_old, const double* __restrict__ bx,
-                             const double* __restrict__ by, const double* __restrict__ bz,
-                             const double* __restrict__ fsx, const double* __restrict__ fsy,
-                             const double* __restrict__ fsz, const uint8_t* __restrict__ cellbits, double* rhs,
-                             double* rhs_ref) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  if (i >= g.nx || j >= g.ny || k >= g.nz) return;
-  const int ix = i + 1, iy = j + 1, iz = k + 1;
-  const int c = g.idx(i, j, k);
-  double out = 0.0;
-  if (cellbits[c] & 1) {
-    double exp_ = 1.0, exm = 1.0, eyp = 1.0, eym = 1.0, ezp = 1.0, ezm = 1.0, deps = 0.0;
-    if (eps) {
-      const double e0 = eps[R.cell(ix, iy, iz)];
-      exp_ = DMUL(0.5, DADD(e0, eps[R.cell(ix + 1, iy, iz)]));
-      exm = DMUL(0.5, DADD(eps[R.cell(ix - 1, iy, iz)], e0));
-      eyp = DMUL(0.5, DADD(e0, eps[R.cell(ix, iy + 1, iz)]));
-      eym = DMUL(0.5, DADD(eps[R.cell(ix, iy - 1, iz)], e0));
-      ezp = DMUL(0.5, DADD(e0, eps[R.cell(ix, iy, iz + 1)]));
-      ezm = DMUL(0.5, DADD(eps[R.cell(ix, iy, iz - 1)], e0));
-      deps = DADD(e0, -eps_old[R.cell(ix, iy, iz)]);
-    }
-    const double tx = DMUL(DADD(DMUL(exp_, vx[R.xf(ix + 1, iy, iz)]), -DMUL(exm, vx[R.xf(ix, iy, iz)])), inv_dx);
-    const double ty = DMUL(DADD(DMUL(eyp, vy[R.yf(ix, iy + 1, iz)]), -DMUL(eym, vy[R.yf(ix, iy, iz)])), inv_dy);
-    const double tz = DMUL(DADD(DMUL(ezp, vz[R.zf(ix, iy, iz + 1)]), -DMUL(ezm, vz[R.zf(ix, iy, iz)])), inv_dz);
-    const double div_eps = DADD(DADD(tx, ty), tz);
-    double f_st = 0.0;
-    if (fsx) {
-      const double sx = DMUL(DADD(DMUL(bx[c + 1], fsx[R.xf(ix + 1, iy, iz)]), -DMUL(bx[c], fsx[R.xf(ix, iy, iz)])), inv_dx);
-      const double sy = DMUL(DADD(DMUL(by[c + g.px], fsy[R.yf(ix, iy + 1, iz)]), -DMUL(by[c], fsy[R.yf(ix, iy, iz)])), inv_dy);
-      const double sz = DMUL(DADD(DMUL(bz[c + g.ps], fsz[R.zf(ix, iy, iz + 1)]), -DMUL(bz[c], fsz[R.zf(ix, iy, iz)])), inv_dz);
-      f_st = DADD(DADD(sx, sy), sz);
-    }
-    out = DADD(DADD(DMUL(-inv_dt, div_eps), -DMUL(DMUL(deps, inv_dt), inv_dt)), -f_st);
-  }
-  rhs[c] = out;
-  if (rhs_ref) rhs_ref[R.cell(ix, iy, iz)] = out;
-}
-
-// The same RHS without ε and f_s (ε = 1, f_s = 0: the same operations with
-// those constants), KZ planes per thread with every plane's loads issued
-// before the first result is formed; a z-face between two of the planes is
-// read once.
-template <int KZ>
-__global__ void __launch_bounds__(TNT) k_divergence_z(Geom g, RefDims R, double inv_dx, double inv_dy, double inv_dz,
-                                                      double inv_dt, const double* __restrict__ vx,
-                                                      const double* __restrict__ vy, const double* __restrict__ vz,
-                                                      const uint8_t* __restrict__ cellbits, double* rhs,
-                                                      double* rhs_ref) {
+// KZ planes per thread, every plane's loads issued before the first result is
+// formed; values between two of the planes are read once.  EPS, FS: with the
+// void fractions, with the surface tension.
+template <int KZ, bool EPS, bool FS>
+__global__ void __launch_bounds__(TNT)
+    k_divergence(Geom g, RefDims R, double inv_dx, double inv_dy, double inv_dz, double inv_dt,
+                 const double* __restrict__ vx, const double* __restrict__ vy, const double* __restrict__ vz,
+                 const double* __restrict__ eps, const double* __restrict__ eps_old, const double* __restrict__ bx,
+                 const double* __restrict__ by, const double* __restrict__ bz, const double* __restrict__ fsx,
+                 const double* __restrict__ fsy, const double* __restrict__ fsz, const uint8_t* __restrict__ cellbits,
+                 double* __restrict__ rhs, double* __restrict__ rhs_ref) {
   const int i = blockIdx.x * TBX + threadIdx.x;
   const int j = blockIdx.y * TBY + threadIdx.y;
   const int k0 = blockIdx.z * KZ;
   if (i >= g.nx || j >= g.ny) return;
   const int ix = i + 1, iy = j + 1;
+  const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2);
   double xp[KZ], xm[KZ], yp[KZ], ym[KZ], zf[KZ + 1];
+  // (EPS) eps at x-+1, y-+1 and in the own column, eps_old; (FS) f_b f_s at the faces, each rounded as the product
+  double ex[EPS ? KZ : 1][2], ey[EPS ? KZ : 1][2], ez[EPS ? KZ + 2 : 1], eo[EPS ? KZ : 1];
+  double sxf[FS ? KZ : 1][2], syf[FS ? KZ : 1][2], szf[FS ? KZ + 1 : 1];
   uint8_t bits[KZ];
 #pragma unroll
   for (int q = 0; q < KZ; ++q) {
     const int k = k0 + q, iz = k + 1;
     bits[q] = 0;
-    xp[q] = xm[q] = yp[q] = ym[q] = 0.0;
+    xp[q] = xm[q] = yp[q] = ym[q] = zf[q] = 0.0;
     if (k < g.nz) {
-      bits[q] = cellbits[g.idx(i, j, k)];
-      xp[q] = vx[R.xf(ix + 1, iy, iz)];
-      xm[q] = vx[R.xf(ix, iy, iz)];
-      yp[q] = vy[R.yf(ix, iy + 1, iz)];
-      ym[q] = vy[R.yf(ix, iy, iz)];
+      const long long fx = R.xf(ix, iy, iz), fy = R.yf(ix, iy, iz);
+      const int c = g.idx(i, j, k);
+      bits[q] = cellbits[c];
+      xp[q] = vx[fx + 1];
+      xm[q] = vx[fx];
+      yp[q] = vy[fy + sx];
+      ym[q] = vy[fy];
+      if (EPS) {
+        const long long e = R.cell(ix, iy, iz);
+        ex[q][0] = eps[e - 1];
+        ex[q][1] = eps[e + 1];
+        ey[q][0] = eps[e - sx];
+        ey[q][1] = eps[e + sx];
+        eo[q] = eps_old[e];
+      }
+      if (FS) {
+        sxf[q][0] = DMUL(bx[c], fsx[fx]);
+        sxf[q][1] = DMUL(bx[c + 1], fsx[fx + 1]);
+        syf[q][0] = DMUL(by[c], fsy[fy]);
+        syf[q][1] = DMUL(by[c + g.px], fsy[fy + sx]);
+      }
     }
-    zf[q] = k <= g.nz ? vz[R.zf(ix, iy, iz)] : 0.0;  // the low face of plane k, the top face of plane k-1
   }
-  zf[KZ] = k0 + KZ <= g.nz ? vz[R.zf(ix, iy, k0 + KZ + 1)] : 0.0;
+#pragma unroll
+  for (int q = 0; q <= KZ; ++q) {  // the low faces of planes k0 .. k0 + KZ
+    if (k0 + q <= g.nz) {
+      const long long f = R.zf(ix, iy, k0 + q + 1);
+      zf[q] = vz[f];
+      if (FS) szf[q] = DMUL(bz[g.idx(i, j, k0 + q)], fsz[f]);
+    }
+  }
+  if (EPS) {
+#pragma unroll
+    for (int q = 0; q < KZ + 2; ++q)  // planes k0 - 1 .. k0 + KZ
+      if (k0 + q <= g.nz + 1) ez[q] = eps[R.cell(ix, iy, k0 + q)];
+  }
 #pragma unroll
   for (int q = 0; q < KZ; ++q) {
     const int k = k0 + q;
     if (k >= g.nz) break;
-    const double ztop = zf[q + 1];
     double out = 0.0;
     if (bits[q] & 1) {
-      const double one = 1.0, deps = 0.0, f_st = 0.0;
-      const double tx = DMUL(DADD(DMUL(one, xp[q]), -DMUL(one, xm[q])), inv_dx);
-      const double ty = DMUL(DADD(DMUL(one, yp[q]), -DMUL(one, ym[q])), inv_dy);
-      const double tz = DMUL(DADD(DMUL(one, ztop), -DMUL(one, zf[q])), inv_dz);
+      double exp_ = 1.0, exm = 1.0, eyp = 1.0, eym = 1.0, ezp = 1.0, ezm = 1.0, deps = 0.0, f_st = 0.0;
+      if (EPS) {
+        const double e0 = ez[q + 1];
+        exp_ = DMUL(0.5, DADD(e0, ex[q][1]));
+        exm = DMUL(0.5, DADD(ex[q][0], e0));
+        eyp = DMUL(0.5, DADD(e0, ey[q][1]));
+        eym = DMUL(0.5, DADD(ey[q][0], e0));
+        ezp = DMUL(0.5, DADD(e0, ez[q + 2]));
+        ezm = DMUL(0.5, DADD(ez[q], e0));
+        deps = DADD(e0, -eo[q]);
+      }
+      const double tx = DMUL(DADD(DMUL(exp_, xp[q]), -DMUL(exm, xm[q])), inv_dx);
+      const double ty = DMUL(DADD(DMUL(eyp, yp[q]), -DMUL(eym, ym[q])), inv_dy);
+      const double tz = DMUL(DADD(DMUL(ezp, zf[q + 1]), -DMUL(ezm, zf[q])), inv_dz);
       const double div_eps = DADD(DADD(tx, ty), tz);
+      if (FS)
+        f_st = DADD(DADD(DMUL(DADD(sxf[q][1], -sxf[q][0]), inv_dx), DMUL(DADD(syf[q][1], -syf[q][0]), inv_dy)),
+                    DMUL(DADD(szf[q + 1], -szf[q]), inv_dz));
       out = DADD(DADD(DMUL(-inv_dt, div_eps), -DMUL(DMUL(deps, inv_dt), inv_dt)), -f_st);
     }
     rhs[g.idx(i, j, k)] = out;
@@ -1180,67 +1180,58 @@ __global__ void __launch_bounds__(1024) k_coarse_vcycle(CoarseSet set, int nu1, 
 // ------------------------------------------------------------------------
 // Velocity correction: k_correct_vof_velocity (CFD/G_SMACSolver.cu:1072-1142),
 // same thread ranges and operation order.  fs == nullptr: f_s = 0;
-// fir == nullptr: f_inv_rho taken from the padded f_b.  write_all: faces that
-// are not F_INTERIOR receive u* (used by smac_project).
-__global__ void k_correct(RefDims R, Geom g, double inv_dx, double inv_dy, double inv_dz, double dt,
-                          const uint8_t* __restrict__ ct, const uint8_t* __restrict__ fxt,
-                          const uint8_t* __restrict__ fyt, const uint8_t* __restrict__ fzt,
-                          const double* __restrict__ pd, double* p, const double* __restrict__ vxs,
-                          const double* __restrict__ vys, const double* __restrict__ vzs,
-                          const double* __restrict__ firx, const double* __restrict__ firy,
-                          const double* __restrict__ firz, const double* __restrict__ fbx,
-                          const double* __restrict__ fby, const double* __restrict__ fbz,
-                          const double* __restrict__ fsx, const double* __restrict__ fsy,
-                          const double* __restrict__ fsz, double* vx, double* vy, double* vz, int write_all) {
-  // every face index from 0 (the reference's threads start at 1; index-0
-  // faces are ghost faces that only write_all touches)
-  const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-  const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+// fir == nullptr: f_inv_rho taken from the padded f_b.  Only F_INTERIOR faces
+// are written (with both of their cells inside: a mislabelled ghost face is
+// left alone).  A face's values are loaded with its type, not after it.
+__global__ void __launch_bounds__(TNT)
+    k_correct(RefDims R, Geom g, double inv_dx, double inv_dy, double inv_dz, double dt,
+              const uint8_t* __restrict__ ct, const uint8_t* __restrict__ fxt, const uint8_t* __restrict__ fyt,
+              const uint8_t* __restrict__ fzt, const double* pd, double* p, const double* vxs, const double* vys,
+              const double* vzs, const double* firx, const double* firy, const double* firz,
+              const double* __restrict__ fbx, const double* __restrict__ fby, const double* __restrict__ fbz,
+              const double* fsx, const double* fsy, const double* fsz, double* vx, double* vy, double* vz) {
+  // indices 0 .. N+1: each family's faces with a cell on both sides
+  const int ix = blockIdx.x * TBX + threadIdx.x;
+  const int iy = blockIdx.y * TBY + threadIdx.y;
   const int iz = blockIdx.z;
   const int Nx = R.Nx, Ny = R.Ny, Nz = R.Nz;
-  // padded f_b of the face, used when f_inv_rho is not supplied
-  auto padded = [&](const double* b, int i, int j, int k) -> double {
-    if (i < 0 || j < 0 || k < 0 || i > g.nx || j > g.ny || k > g.nz) return 0.0;
-    return b[g.idx(i, j, k)];
-  };
-  // a face is corrected only when both of its cells exist (F_INTERIOR faces
-  // always satisfy this; the bound keeps mislabelled ghost faces harmless)
-  if (!(iy >= Ny + 2 || ix >= Nx + 3 || iz >= Nz + 2)) {
-    const long long f = R.xf(ix, iy, iz);
-    if (fxt[f] == F_INTERIOR && ix >= 1 && ix <= Nx + 1) {
-      const double ir = firx ? firx[f] : padded(fbx, ix - 1, iy - 1, iz - 1);
-      const double fs = fsx ? fsx[f] : 0.0;
-      const double gp = DMUL(DADD(pd[R.cell(ix, iy, iz)], -pd[R.cell(ix - 1, iy, iz)]), inv_dx);
-      vx[f] = DADD(vxs[f], DMUL(DMUL(ir, dt), DADD(fs, -gp)));
-    } else if (write_all) {
-      vx[f] = vxs[f];
-    }
+  if (ix > Nx + 1 || iy > Ny + 1) return;
+  const long long sx = Nx + 2, sxy = sx * (Ny + 2), c = R.cell(ix, iy, iz);
+  const long long fx = R.xf(ix, iy, iz), fy = R.yf(ix, iy, iz), fz = R.zf(ix, iy, iz);
+  const bool xr = ix >= 1, yr = iy >= 1, zr = iz >= 1, in = xr && yr && zr;
+  const int pc = in ? g.idx(ix - 1, iy - 1, iz - 1) : 0;  // the padded f_b of the faces (0 on the low ghost layers)
+  const double p0 = pd[c];
+  const uint8_t tc = ct[c];
+  double px = 0.0, py = 0.0, pz = 0.0, ux = 0.0, uy = 0.0, uz = 0.0, ax = 0.0, ay = 0.0, az = 0.0, bx = 0.0, by = 0.0,
+         bz = 0.0;
+  uint8_t tx = F_GHOST, ty = F_GHOST, tz = F_GHOST;
+  if (xr) {
+    px = pd[c - 1];
+    tx = fxt[fx];
+    ux = vxs[fx];
+    ax = firx ? firx[fx] : in ? fbx[pc] : 0.0;
+    if (fsx) bx = fsx[fx];
   }
-  if (!(iy >= Ny + 3 || ix >= Nx + 2 || iz >= Nz + 2)) {
-    const long long f = R.yf(ix, iy, iz);
-    if (fyt[f] == F_INTERIOR && iy >= 1 && iy <= Ny + 1) {
-      const double ir = firy ? firy[f] : padded(fby, ix - 1, iy - 1, iz - 1);
-      const double fs = fsy ? fsy[f] : 0.0;
-      const double gp = DMUL(DADD(pd[R.cell(ix, iy, iz)], -pd[R.cell(ix, iy - 1, iz)]), inv_dy);
-      vy[f] = DADD(vys[f], DMUL(DMUL(ir, dt), DADD(fs, -gp)));
-    } else if (write_all) {
-      vy[f] = vys[f];
-    }
+  if (yr) {
+    py = pd[c - sx];
+    ty = fyt[fy];
+    uy = vys[fy];
+    ay = firy ? firy[fy] : in ? fby[pc] : 0.0;
+    if (fsy) by = fsy[fy];
   }
-  if (!(iy >= Ny + 2 || ix >= Nx + 2 || iz >= Nz + 3)) {
-    const long long f = R.zf(ix, iy, iz);
-    if (fzt[f] == F_INTERIOR && iz >= 1 && iz <= Nz + 1) {
-      const double ir = firz ? firz[f] : padded(fbz, ix - 1, iy - 1, iz - 1);
-      const double fs = fsz ? fsz[f] : 0.0;
-      const double gp = DMUL(DADD(pd[R.cell(ix, iy, iz)], -pd[R.cell(ix, iy, iz - 1)]), inv_dz);
-      vz[f] = DADD(vzs[f], DMUL(DMUL(ir, dt), DADD(fs, -gp)));
-    } else if (write_all) {
-      vz[f] = vzs[f];
-    }
+  if (zr) {
+    pz = pd[c - sxy];
+    tz = fzt[fz];
+    uz = vzs[fz];
+    az = firz ? firz[fz] : in ? fbz[pc] : 0.0;
+    if (fsz) bz = fsz[fz];
   }
-  if (p && ix >= 1 && iy >= 1 && iz >= 1 && ix < Nx + 1 && iy < Ny + 1 && iz < Nz + 1) {
-    if (ct[R.cell(ix, iy, iz)] == C_INTERIOR) p[R.cell(ix, iy, iz)] = DADD(p[R.cell(ix, iy, iz)], pd[R.cell(ix, iy, iz)]);
-  }
+  const bool cell = p && in && ix <= Nx && iy <= Ny && iz <= Nz;
+  const double pold = cell ? p[c] : 0.0;
+  if (tx == F_INTERIOR) vx[fx] = DADD(ux, DMUL(DMUL(ax, dt), DADD(bx, -DMUL(DADD(p0, -px), inv_dx))));
+  if (ty == F_INTERIOR) vy[fy] = DADD(uy, DMUL(DMUL(ay, dt), DADD(by, -DMUL(DADD(p0, -py), inv_dy))));
+  if (tz == F_INTERIOR) vz[fz] = DADD(uz, DMUL(DMUL(az, dt), DADD(bz, -DMUL(DADD(p0, -pz), inv_dz))));
+  if (cell && tc == C_INTERIOR) p[c] = DADD(pold, p0);
 }
 
 // The correction as smac_project runs it (f_s = 0, f_inv_rho from the padded
