@@ -583,43 +583,76 @@ __device__ __forceinline__ double st_diff(bool p, bool m, double fp, double f0, 
   return 0.0;
 }
 
+// Planes per thread of the two passes, whose loads are issued together: with
+// one, k_st_force took 113 us at 192^3, with two 97; the explicit half there
+// 1242, 1223, 1215 and 1228 us with one in the old form, one, two and four.
+constexpr int ST_KZ = 2;
+
 // Pass 1, k_calc_interface_normal (:87-182): grad alpha, |grad alpha| and the
 // unit normal of every C_INTERIOR cell; other cells are left as they are.
 __global__ void __launch_bounds__(256) k_st_normal(StArgs A) {
   const RefDims& R = A.R;
-  const int ix = blockIdx.x * 32 + threadIdx.x + 1, iy = blockIdx.y * 8 + threadIdx.y + 1, iz = blockIdx.z + 1;
+  const int ix = blockIdx.x * 32 + threadIdx.x + 1, iy = blockIdx.y * 8 + threadIdx.y + 1;
+  const int iz0 = blockIdx.z * ST_KZ + 1;
   if (ix > R.Nx || iy > R.Ny) return;
-  const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2), c = R.cell(ix, iy, iz);
-  if (A.ct[c] != kInterior) return;
-  const double* a = A.alpha;
-  const double gx = st_diff(A.ct[c + 1] == kInterior, A.ct[c - 1] == kInterior, a[c + 1], a[c], a[c - 1], A.i2h[0],
-                            A.ih[0]);
-  const double gy = st_diff(A.ct[c + sx] == kInterior, A.ct[c - sx] == kInterior, a[c + sx], a[c], a[c - sx],
-                            A.i2h[1], A.ih[1]);
-  const double gz = st_diff(A.ct[c + sxy] == kInterior, A.ct[c - sxy] == kInterior, a[c + sxy], a[c], a[c - sxy],
-                            A.i2h[2], A.ih[2]);
-  const double mag2 = DADD(DADD(DMUL(gx, gx), DMUL(gy, gy)), DMUL(gz, gz));
-  const double mag = __dsqrt_rn(mag2);
-  A.gm[c] = mag;
-  if (mag2 > 1e-12) {
-    const double inv = __ddiv_rn(1.0, mag);
-    A.nx[c] = DMUL(gx, inv);
-    A.ny[c] = DMUL(gy, inv);
-    A.nz[c] = DMUL(gz, inv);
-  } else {
-    A.nx[c] = 0.0;
-    A.ny[c] = 0.0;
-    A.nz[c] = 0.0;
+  const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2), c0 = R.cell(ix, iy, iz0);
+  const double* __restrict__ a = A.alpha;
+  const uint8_t* __restrict__ ct = A.ct;
+  double az[ST_KZ + 2], ax[ST_KZ][2], ay[ST_KZ][2];
+  uint8_t tz[ST_KZ + 2], tx[ST_KZ][2], ty[ST_KZ][2];
+#pragma unroll
+  for (int q = 0; q < ST_KZ + 2; ++q) {  // the own column, planes iz0 - 1 .. iz0 + KZ
+    az[q] = 0.0;
+    tz[q] = 2;
+    if (iz0 + q - 1 <= R.Nz + 1) {
+      az[q] = a[c0 + (q - 1) * sxy];
+      tz[q] = ct[c0 + (q - 1) * sxy];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < ST_KZ; ++q) {
+    const long long c = c0 + q * sxy;
+    if (iz0 + q > R.Nz) break;
+    ax[q][0] = a[c - 1];
+    ax[q][1] = a[c + 1];
+    ay[q][0] = a[c - sx];
+    ay[q][1] = a[c + sx];
+    tx[q][0] = ct[c - 1];
+    tx[q][1] = ct[c + 1];
+    ty[q][0] = ct[c - sx];
+    ty[q][1] = ct[c + sx];
+  }
+#pragma unroll
+  for (int q = 0; q < ST_KZ; ++q) {
+    const long long c = c0 + q * sxy;
+    if (iz0 + q > R.Nz) break;
+    if (tz[q + 1] != kInterior) continue;
+    const double ac = az[q + 1];
+    const double gx = st_diff(tx[q][1] == kInterior, tx[q][0] == kInterior, ax[q][1], ac, ax[q][0], A.i2h[0], A.ih[0]);
+    const double gy = st_diff(ty[q][1] == kInterior, ty[q][0] == kInterior, ay[q][1], ac, ay[q][0], A.i2h[1], A.ih[1]);
+    const double gz = st_diff(tz[q + 2] == kInterior, tz[q] == kInterior, az[q + 2], ac, az[q], A.i2h[2], A.ih[2]);
+    const double mag2 = DADD(DADD(DMUL(gx, gx), DMUL(gy, gy)), DMUL(gz, gz));
+    const double mag = __dsqrt_rn(mag2);
+    A.gm[c] = mag;
+    double nx = 0.0, ny = 0.0, nz = 0.0;
+    if (mag2 > 1e-12) {
+      const double inv = __ddiv_rn(1.0, mag);
+      nx = DMUL(gx, inv);
+      ny = DMUL(gy, inv);
+      nz = DMUL(gz, inv);
+    }
+    A.nx[c] = nx;
+    A.ny[c] = ny;
+    A.nz[c] = nz;
   }
 }
 
-// Curvature of cell (ix,iy,iz) in 1..N, k_calc_curvature (:184-290):
+// Curvature of cell c (in 1..N) with alpha a, k_calc_curvature (:184-290):
 // 0 outside 0.01 <= alpha <= 0.99, else -div n, a neighbour counting where
 // it is C_INTERIOR with |grad alpha| > 1e-6.
-__device__ double st_kappa(const StArgs& A, int ix, int iy, int iz) {
+__device__ double st_kappa(const StArgs& A, long long c, double a) {
   const RefDims& R = A.R;
-  const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2), c = R.cell(ix, iy, iz);
-  const double a = A.alpha[c];
+  const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2);
   if (a > 0.99 || a < 0.01) return 0.0;
   auto ok = [&](long long n) { return A.ct[n] == kInterior && A.gm[n] > 1e-6; };
   const double dnx = st_diff(ok(c + 1), ok(c - 1), A.nx[c + 1], A.nx[c], A.nx[c - 1], A.i2h[0], A.ih[0]);
@@ -638,57 +671,93 @@ __device__ __forceinline__ double st_force(double sigma, double ap, double am, d
 
 constexpr int ST_TX = 32, ST_TY = 8;
 
-// Pass 2: curvature and face force fused.  A block owns a 32 x 8 tile of one
-// plane: each thread computes its cell's curvature (stored) and the one
-// below it, 40 threads also the tile's low-x column and low-y row (into a
-// shared tile), and after one barrier every thread writes the three faces on
-// the low side of its cell.  Cells with alpha outside [0.01, 0.99], most of
-// them, cost one load per curvature, so the recomputation is cheap; a
-// z-march that carried the curvature below in a register ran at a quarter of
-// the occupancy (one barrier per plane, serial planes) and took 2.5x as long.
+// Pass 2: curvature and face force fused.  A block owns a 32 x 8 tile of ST_KZ
+// planes: each thread computes its cells' curvatures (stored) and the one
+// below the first, 40 threads per plane those of the tile's low-x column and
+// low-y row (into a shared tile), and after one barrier every thread writes
+// the three faces on the low side of its cells.  Cells with alpha outside
+// [0.01, 0.99], most of them, cost one load per curvature, so the
+// recomputation is cheap; a z-march that carried the curvature below in a
+// register, with a barrier per plane, took 2.5x as long.
 // Faces 1..N of every family are written (0 where the reference's memset
 // leaves 0); the rest is k_st_rim's.
-__global__ void __launch_bounds__(ST_TX* ST_TY, 4) k_st_force(StArgs A) {
-  __shared__ double ks[ST_TY + 1][ST_TX + 1];
+__global__ void __launch_bounds__(ST_TX* ST_TY) k_st_force(StArgs A) {
+  __shared__ double ks[ST_KZ][ST_TY + 1][ST_TX + 1];
   const RefDims& R = A.R;
   const int tx = threadIdx.x, ty = threadIdx.y, t = ty * ST_TX + tx;
-  const int x0 = blockIdx.x * ST_TX, y0 = blockIdx.y * ST_TY, iz = blockIdx.z + 1;
+  const int x0 = blockIdx.x * ST_TX, y0 = blockIdx.y * ST_TY, iz0 = blockIdx.z * ST_KZ + 1;
   const int ix = x0 + tx + 1, iy = y0 + ty + 1;
   const bool in = ix <= R.Nx && iy <= R.Ny;
-  // the extra cell: column x0 (rows y0+1..y0+8) or row y0 (columns x0+1..x0+32)
-  const bool hcol = t < ST_TY, hrow = t >= ST_TY && t < ST_TY + ST_TX;
-  const int hx = hcol ? x0 : x0 + 1 + (t - ST_TY), hy = hcol ? y0 + 1 + t : y0;
-  const bool hin = (hcol || hrow) && hx >= 1 && hx <= R.Nx && hy >= 1 && hy <= R.Ny;
   const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2);
-  double k = 0.0, kb = 0.0, a0 = 0.0, ax = 0.0, ay = 0.0, az = 0.0;
-  bool fx = false, fy = false, fz = false;
-  long long c = 0;
+  const double* __restrict__ al = A.alpha;
+  const uint8_t* __restrict__ ct = A.ct;
+  double k[ST_KZ], a[ST_KZ + 1], ax[ST_KZ], ay[ST_KZ], kb = 0.0;
+  bool fx[ST_KZ], fy[ST_KZ], fz[ST_KZ];
+  const long long c0 = in ? R.cell(ix, iy, iz0) : 0;
   if (in) {
     // everything the faces need but the shared tile, before the barrier
-    c = R.cell(ix, iy, iz);
-    const bool c0 = A.ct[c] == kInterior;
-    fx = ix >= 2 && c0 && A.ct[c - 1] == kInterior;
-    fy = iy >= 2 && c0 && A.ct[c - sx] == kInterior;
-    fz = iz >= 2 && c0 && A.ct[c - sxy] == kInterior;
-    a0 = A.alpha[c];
-    ax = A.alpha[c - 1];
-    ay = A.alpha[c - sx];
-    az = A.alpha[c - sxy];
-    k = st_kappa(A, ix, iy, iz);
-    if (fz) kb = st_kappa(A, ix, iy, iz - 1);
-    A.kappa[c] = k;
+    uint8_t tc[ST_KZ + 1], tl[ST_KZ][2];
+#pragma unroll
+    for (int q = 0; q <= ST_KZ; ++q) {  // the own column, planes iz0 - 1 .. iz0 + KZ - 1
+      a[q] = 0.0;
+      tc[q] = 2;
+      if (iz0 + q - 1 <= R.Nz) {
+        a[q] = al[c0 + (q - 1) * sxy];
+        tc[q] = ct[c0 + (q - 1) * sxy];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < ST_KZ; ++q) {
+      const long long c = c0 + q * sxy;
+      ax[q] = ay[q] = 0.0;
+      tl[q][0] = tl[q][1] = 2;
+      if (iz0 + q <= R.Nz) {
+        ax[q] = al[c - 1];
+        ay[q] = al[c - sx];
+        tl[q][0] = ct[c - 1];
+        tl[q][1] = ct[c - sx];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < ST_KZ; ++q) {
+      const bool i0 = tc[q + 1] == kInterior;
+      fx[q] = ix >= 2 && i0 && tl[q][0] == kInterior;
+      fy[q] = iy >= 2 && i0 && tl[q][1] == kInterior;
+      fz[q] = iz0 + q >= 2 && i0 && tc[q] == kInterior;
+      k[q] = 0.0;
+      if (iz0 + q <= R.Nz) {
+        k[q] = st_kappa(A, c0 + q * sxy, a[q + 1]);
+        A.kappa[c0 + q * sxy] = k[q];
+      }
+    }
+    if (fz[0]) kb = st_kappa(A, c0 - sxy, a[0]);
   }
-  ks[ty + 1][tx + 1] = k;
-  if (hcol || hrow) {
-    const double kh = hin ? st_kappa(A, hx, hy, iz) : 0.0;
-    if (hcol) ks[t + 1][0] = kh;
-    else ks[0][t - ST_TY + 1] = kh;
+#pragma unroll
+  for (int q = 0; q < ST_KZ; ++q) ks[q][ty + 1][tx + 1] = in ? k[q] : 0.0;
+  // the extra cells: column x0 (rows y0+1..y0+8) or row y0 (columns x0+1..x0+32) of each plane
+  for (int e = t; e < ST_KZ * (ST_TX + ST_TY); e += ST_TX * ST_TY) {
+    const int q = e / (ST_TX + ST_TY), u = e - q * (ST_TX + ST_TY);
+    const bool col = u < ST_TY;
+    const int hx = col ? x0 : x0 + 1 + (u - ST_TY), hy = col ? y0 + 1 + u : y0;
+    double kh = 0.0;
+    if (hx >= 1 && hx <= R.Nx && hy >= 1 && hy <= R.Ny && iz0 + q <= R.Nz) {
+      const long long c = R.cell(hx, hy, iz0 + q);
+      kh = st_kappa(A, c, al[c]);
+    }
+    if (col) ks[q][u + 1][0] = kh;
+    else ks[q][0][u - ST_TY + 1] = kh;
   }
   __syncthreads();
   if (!in) return;
-  A.fs[0][R.xf(ix, iy, iz)] = fx ? st_force(A.sigma, a0, ax, k, ks[ty + 1][tx], A.ih[0]) : 0.0;
-  A.fs[1][R.yf(ix, iy, iz)] = fy ? st_force(A.sigma, a0, ay, k, ks[ty][tx + 1], A.ih[1]) : 0.0;
-  A.fs[2][R.zf(ix, iy, iz)] = fz ? st_force(A.sigma, a0, az, k, kb, A.ih[2]) : 0.0;
+#pragma unroll
+  for (int q = 0; q < ST_KZ; ++q) {
+    const int iz = iz0 + q;
+    if (iz > R.Nz) break;
+    const double kz = q ? k[q > 0 ? q - 1 : 0] : kb;
+    A.fs[0][R.xf(ix, iy, iz)] = fx[q] ? st_force(A.sigma, a[q + 1], ax[q], k[q], ks[q][ty + 1][tx], A.ih[0]) : 0.0;
+    A.fs[1][R.yf(ix, iy, iz)] = fy[q] ? st_force(A.sigma, a[q + 1], ay[q], k[q], ks[q][ty][tx + 1], A.ih[1]) : 0.0;
+    A.fs[2][R.zf(ix, iy, iz)] = fz[q] ? st_force(A.sigma, a[q + 1], a[q], k[q], kz, A.ih[2]) : 0.0;
+  }
 }
 
 // Zero of every face outside the box 1..N of each family (the part of the
@@ -1647,8 +1716,9 @@ smac_status smac_surface_tension(const smac_grid_desc* d, const double* alpha, c
   cudaStream_t s = (cudaStream_t)stream;
   const unsigned bx = (unsigned)((d->nx + ST_TX - 1) / ST_TX), by = (unsigned)((d->ny + ST_TY - 1) / ST_TY);
   k_st_rim<<<dim3(64, 9), 256, 0, s>>>(A);
-  k_st_normal<<<dim3(bx, by, (unsigned)d->nz), dim3(32, 8), 0, s>>>(A);
-  k_st_force<<<dim3(bx, by, (unsigned)d->nz), dim3(ST_TX, ST_TY), 0, s>>>(A);
+  const unsigned bz = (unsigned)((d->nz + ST_KZ - 1) / ST_KZ);
+  k_st_normal<<<dim3(bx, by, bz), dim3(32, 8), 0, s>>>(A);
+  k_st_force<<<dim3(bx, by, bz), dim3(ST_TX, ST_TY), 0, s>>>(A);
   return launch_status(fn);
 }
 
