@@ -385,7 +385,12 @@ void launch_zm_shape(smac_handle* h, int l, const T* xin, T* xout, const T* rhs,
   long long best = -1;
   // (an item costs about six steps beyond its planes: two extra c0 planes and
   // the exposed latency of its first loads; measured at 192^3 and 256^3)
-  for (int cand = std::min(64, g.nz); cand >= std::min(4, g.nz); --cand) {
+  // Down to one plane: a grid too small for an item per CTA then ends in the
+  // fewest steps (with at least four planes an item, 64^3 had 176 items for
+  // 444 CTAs; projections of 32^3 FP64, 64^3, 150 x 100 x 75 and 256^3 mixed
+  // took 615, 796, 1581 and 5727 us, 572, 770, 1524 and 5680 with two, 553,
+  // 770, 1528 and 5679 with one).
+  for (int cand = std::min(64, g.nz); cand >= 1; --cand) {
     const long long items = nty * ((g.nz + cand - 1) / cand);
     const long long cost = ((items + slots - 1) / slots) * (cand + 6);
     if (best < 0 || cost < best) { best = cost; zc = cand; }
