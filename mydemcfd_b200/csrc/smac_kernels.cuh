@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(TNT)
   const int k0 = blockIdx.z * KZ;
   if (i >= g.nx || j >= g.ny) return;
   const int ix = i + 1, iy = j + 1;
-  const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2);
+  const long long sx = R.Nx + 2;
   double xp[KZ], xm[KZ], yp[KZ], ym[KZ], zf[KZ + 1];
   // (EPS) eps at x-+1, y-+1 and in the own column, eps_old; (FS) f_b f_s at the faces, each rounded as the product
   double ex[EPS ? KZ : 1][2], ey[EPS ? KZ : 1][2], ez[EPS ? KZ + 2 : 1], eo[EPS ? KZ : 1];
