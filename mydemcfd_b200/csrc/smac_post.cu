@@ -1010,9 +1010,10 @@ __device__ __forceinline__ double m_vstar(const MomArgs& A, const int* b) {
   return DMUL(DSUB(1.0, A.sf[AF] ? A.sf[AF][f] : 0.0), vs);
 }
 
-// The predictor kernel.  A face is regular when every face of the three
-// families within two indices of it is F_INTERIOR (so nothing it reads passes
-// through a boundary rule); all but a shell of the box and around solids are.
+// The predictor kernel.  A face is regular when every face of its family
+// within two indices of it and every face of the other two within one is
+// F_INTERIOR (its stencil reads no further, so nothing it reads passes through
+// a boundary rule); all but a shell of the box and around solids are.
 // For regular faces u* is a sum of differences of side terms, the stress and
 // the convective flux through the control volume's sides, and a minus side's
 // terms are the plus side's of the neighbour bit for bit (the same products
@@ -1190,8 +1191,8 @@ __global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_vstar(const __grid
   const bool own = lane >= 1 && x <= N0 + 1 && y <= N1 + 1;
   if (tid == 0) qcount = 0;
 
-  // The types around the chunk, OR-ed over the families (1 outside the
-  // arrays): planes z0-2 .. z1+1.
+  // Bit F of an entry: family F's face there is not F_INTERIOR (all three
+  // outside the arrays).  Planes z0-2 .. z1+1.
   bool any = false;
   const int np = z1 - z0 + 4;
 #pragma unroll
@@ -1203,31 +1204,46 @@ __global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_vstar(const __grid
 #pragma unroll 4
     for (int p = 0; p < np; ++p) {
       const int gz = z0 - 2 + p;
-      uint32_t t = 1;
+      uint32_t t = 7;
       if (in && gz >= 0 && gz <= N2 + 1)
-        t = A.ft[0][o0 + gz * A.st[0][2]] | A.ft[1][o1 + gz * A.st[1][2]] | A.ft[2][o2 + gz * A.st[2][2]];
+        t = (A.ft[0][o0 + gz * A.st[0][2]] != 0) | (A.ft[1][o1 + gz * A.st[1][2]] != 0) << 1 |
+            (A.ft[2][o2 + gz * A.st[2][2]] != 0) << 2;
       types[p][e] = (uint8_t)t;
       any |= t != 0;
     }
   }
-  // bit p: a type other than F_INTERIOR within two rows and columns on plane z0 - 2 + p
-  uint32_t near = 0;
+  // bit p, plane z0 - 2 + p: such a face of the own family within two rows and
+  // columns (near2), of another family within one (near1)
+  uint32_t near2 = 0, near1 = 0;
   if (__syncthreads_or(any)) {
+    const uint32_t mine_bit = 1u << fam;
     for (int p = 0; p < np; ++p) {
-      uint32_t a = 0, b = 0;
+      // ORs over the rows around the own one, columns lane and 32 + lane (lanes 0..3)
+      uint32_t a2 = 0, b2 = 0, a1 = 0, b1 = 0;
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
-        a |= types[p][(row + r) * PV_FC + lane];
-        if (lane < 4) b |= types[p][(row + r) * PV_FC + 32 + lane];
+        const uint32_t a = types[p][(row + r) * PV_FC + lane];
+        const uint32_t b = lane < 4 ? types[p][(row + r) * PV_FC + 32 + lane] : 0u;
+        a2 |= a & mine_bit;
+        b2 |= b & mine_bit;
+        if (r >= 1 && r <= 3) {
+          a1 |= a & ~mine_bit;
+          b1 |= b & ~mine_bit;
+        }
       }
-      const unsigned long long m = __ballot_sync(0xffffffffu, a != 0) |
-                                   ((unsigned long long)__ballot_sync(0xffffffffu, b != 0) << 32);
-      near |= (((m >> max(lane - 1, 0)) & 0x1f) ? 1u : 0u) << p;
+      const unsigned long long m2 = __ballot_sync(0xffffffffu, a2 != 0) |
+                                    ((unsigned long long)__ballot_sync(0xffffffffu, b2 != 0) << 32);
+      const unsigned long long m1 = __ballot_sync(0xffffffffu, a1 != 0) |
+                                    ((unsigned long long)__ballot_sync(0xffffffffu, b1 != 0) << 32);
+      // (the own column is lane + 1)
+      near2 |= (((m2 >> max(lane - 1, 0)) & 0x1f) ? 1u : 0u) << p;
+      near1 |= (((m1 >> lane) & 0x7) ? 1u : 0u) << p;
     }
   }
   const uint32_t planes = (1u << (z1 - z0)) - 1u;
   const uint32_t mine = own ? planes : 0u;
-  const uint32_t regular = fast ? mine & ~(near | near >> 1 | near >> 2 | near >> 3 | near >> 4) : 0u;
+  const uint32_t near = near2 | near2 >> 1 | near2 >> 2 | near2 >> 3 | near2 >> 4 | near1 >> 1 | near1 >> 2 | near1 >> 3;
+  const uint32_t regular = fast ? mine & ~near : 0u;
   // the others, queued: a warp takes its planes in turn
   for (uint32_t w = __reduce_or_sync(0xffffffffu, mine & ~regular); w; w &= w - 1) {
     const int p = __ffs(w) - 1;
