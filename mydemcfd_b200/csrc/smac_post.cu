@@ -1010,10 +1010,37 @@ __device__ __forceinline__ double m_vstar(const MomArgs& A, const int* b) {
   return DMUL(DSUB(1.0, A.sf[AF] ? A.sf[AF][f] : 0.0), vs);
 }
 
-// The predictor kernel.  A face is regular when every face of its family
-// within two indices of it and every face of the other two within one is
-// F_INTERIOR (its stencil reads no further, so nothing it reads passes through
-// a boundary rule); all but a shell of the box and around solids are.
+// The predictor, one thread per face index (x, y) of plane z of the box
+// 1..N+1: every face at once, each by m_vstar.  blockIdx.z takes two planes of
+// family 0, the same two of family 1, then of family 2, so that the families
+// share the arrays they all read through L2 while an SM mostly runs one
+// family's code.  It waits on chains of dependent loads (a face type, then the
+// value it selects): resident warps matter more than registers, 5 blocks per
+// SM.  The form of small grids (predict_vstar): 32^3 in 13 us, where the march
+// below takes 29.
+constexpr int PF_BLOCKS = 5, PF_WAVES = 7;
+template <bool TW>
+__global__ void __launch_bounds__(256, PF_BLOCKS) k_predict_faces(const __grid_constant__ MomArgs A) {
+  const int fam = blockIdx.z % 6 / 2;
+  const int x = blockIdx.x * 32 + threadIdx.x + 1, y = blockIdx.y * 8 + threadIdx.y + 1;
+  const int z = blockIdx.z / 6 * 2 + blockIdx.z % 2 + 1;
+  if (x > A.N[0] + 1 || y > A.N[1] + 1 || z > A.N[2] + 1) return;
+  int b[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) b[k] = x + y * A.st[k][1] + z * A.st[k][2];
+  if (fam == 0) {
+    if (A.ft[0][b[0]] == 0) A.vs[0][b[0]] = m_vstar<0, TW>(A, b);
+  } else if (fam == 1) {
+    if (A.ft[1][b[1]] == 0) A.vs[1][b[1]] = m_vstar<1, TW>(A, b);
+  } else {
+    if (A.ft[2][b[2]] == 0) A.vs[2][b[2]] = m_vstar<2, TW>(A, b);
+  }
+}
+
+// The predictor of larger grids.  A face is regular when every face of its
+// family within two indices of it and every face of the other two within one
+// is F_INTERIOR (its stencil reads no further, so nothing it reads passes
+// through a boundary rule); all but a shell of the box and around solids are.
 // For regular faces u* is a sum of differences of side terms, the stress and
 // the convective flux through the control volume's sides, and a minus side's
 // terms are the plus side's of the neighbour bit for bit (the same products
@@ -1021,24 +1048,17 @@ __device__ __forceinline__ double m_vstar(const MomArgs& A, const int* b) {
 // the edge means coincide).  So a block takes one family's faces of a tile of
 // 31 x 8 indices and a chunk of planes, finds the regular ones from the types
 // (read once per chunk), marches them in z without a type or a branch
-// (m_march), and evaluates the rest from a queue with the boundary rules
-// (m_vstar), all lanes busy.
+// (m_march), and evaluates the other F_INTERIOR ones from a queue with the
+// boundary rules (m_vstar), all lanes busy.
 //
-// Measured at 256^3 (a two-phase step's fields): 1.60 ms; before, with every
-// face evaluating both sides and a type loaded beside each value, 2.34 ms,
-// bound by dependent loads and instruction misses.  It is now bound by the
-// latency of the march's loads, of which 43% hit L1, at the 32 warps per SM
-// that 64 registers allow (46% of the issue slots, 22% of the FP64 pipe; the
-// queue is 0.25 ms of it).  Not kept: blocks of 3 or 5 per SM (1.90, 1.69);
-// chunks of 6, 8 or 14 planes (1.57, 1.57, 1.70; 192^3 likes 10: 1.24 against
-// 1.29, 1.27, 1.28 for its whole explicit half); a group of warps per family
-// in one block, so that the arrays come through L1 once (1.70 to 1.82); one
-// thread per index for the three families, marching over planes staged in
-// shared memory by 8-byte asynchronous copies, the y-sides exchanged there
-// (2.05: 16 warps per SM and a barrier per plane); the same reading through
-// L1 (2.58); prefetches into L1 or L2 a plane ahead (1.58).
+// Bound by the latency of the march's loads at the 32 warps per SM that 64
+// registers allow (46% of the issue slots, 22% of the FP64 pipe at 256^3):
+// 1.60 ms at 256^3, 2.34 with k_predict_faces.  Blocks of 3 or 5 per SM took
+// 1.90 and 1.69 there, chunks of 6, 8 and 14 planes 1.57, 1.57 and 1.70 (192^3
+// runs fastest with 10: 658 us against 737 and 700 with 6 and 8).
 constexpr int PV_X = 31, PV_Y = 8, PV_NT = 32 * PV_Y, PV_ZMAX = 10, PV_BLOCKS = 4;
 constexpr int PV_FC = 36, PV_FR = PV_Y + 4;  // the type tile: columns x0-2 .. x0+33, rows y0-2 .. y0+PV_Y+1
+static_assert(PV_Y == 8, "both predictor kernels have blocks of 32 x 8");
 static_assert(PV_ZMAX + 4 <= 32 && PV_ZMAX * PV_Y * 32 <= 65536, "plane bits and 16-bit queue entries");
 
 // MUSCL/minmod flux through the side between v0 and np (the values before and
@@ -1159,7 +1179,7 @@ __device__ __forceinline__ void m_march(const MomArgs& A, int x, int y, int z0, 
   }
 }
 
-// The indices in the block's queue, evaluated with the boundary rules.
+// The F_INTERIOR faces in the block's queue, evaluated with the boundary rules.
 template <int AF, bool TW>
 __device__ __forceinline__ void m_queue(const MomArgs& A, const uint16_t* queue, int count, int x0, int y0, int z0) {
   for (int e = threadIdx.y * 32 + threadIdx.x; e < count; e += PV_NT) {
@@ -1168,17 +1188,17 @@ __device__ __forceinline__ void m_queue(const MomArgs& A, const uint16_t* queue,
     int b[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) b[k] = x + y * A.st[k][1] + z * A.st[k][2];
-    if (A.ft[AF][b[AF]] == 0) A.vs[AF][b[AF]] = m_vstar<AF, TW>(A, b);
+    A.vs[AF][b[AF]] = m_vstar<AF, TW>(A, b);
   }
 }
 
 // blockIdx.z: chunk of zc planes (<= PV_ZMAX) and family, families fastest, so
 // that the three families of a chunk share the arrays they all read through
-// L2.  fast: every extent is at least 4 (else no face is regular and the
-// clamped indices would not exist).
+// L2.  fast: every extent is at least 4 (else the march's clamped indices would
+// not exist).
 template <bool TW>
-__global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_vstar(const __grid_constant__ MomArgs A, int zc,
-                                                                         int fast) {
+__global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_march(const __grid_constant__ MomArgs A, int zc,
+                                                                     int fast) {
   __shared__ uint8_t types[PV_ZMAX + 4][PV_FR * PV_FC];
   __shared__ uint16_t queue[PV_X * PV_Y * PV_ZMAX];
   __shared__ int qcount;
@@ -1213,8 +1233,9 @@ __global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_vstar(const __grid
     }
   }
   // bit p, plane z0 - 2 + p: such a face of the own family within two rows and
-  // columns (near2), of another family within one (near1)
-  uint32_t near2 = 0, near1 = 0;
+  // columns (near2), of another family within one (near1), the own face itself
+  // (other)
+  uint32_t near2 = 0, near1 = 0, other = 0;
   if (__syncthreads_or(any)) {
     const uint32_t mine_bit = 1u << fam;
     for (int p = 0; p < np; ++p) {
@@ -1238,16 +1259,20 @@ __global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_predict_vstar(const __grid
       // (the own column is lane + 1)
       near2 |= (((m2 >> max(lane - 1, 0)) & 0x1f) ? 1u : 0u) << p;
       near1 |= (((m1 >> lane) & 0x7) ? 1u : 0u) << p;
+      other |= ((types[p][(row + 2) * PV_FC + lane + 1] & mine_bit) ? 1u : 0u) << p;
     }
   }
   const uint32_t planes = (1u << (z1 - z0)) - 1u;
   const uint32_t mine = own ? planes : 0u;
   const uint32_t near = near2 | near2 >> 1 | near2 >> 2 | near2 >> 3 | near2 >> 4 | near1 >> 1 | near1 >> 2 | near1 >> 3;
   const uint32_t regular = fast ? mine & ~near : 0u;
-  // the others, queued: a warp takes its planes in turn
-  for (uint32_t w = __reduce_or_sync(0xffffffffu, mine & ~regular); w; w &= w - 1) {
+  // the other F_INTERIOR ones, queued: a warp takes its planes in turn (faces
+  // inside solids stay out: with three spheres of a seventh of the grid's
+  // extent, 80^3 takes 101 us, with them in the queue 111)
+  const uint32_t queued = mine & ~regular & ~(other >> 2);
+  for (uint32_t w = __reduce_or_sync(0xffffffffu, queued); w; w &= w - 1) {
     const int p = __ffs(w) - 1;
-    const bool odd = ((mine & ~regular) >> p) & 1u;
+    const bool odd = (queued >> p) & 1u;
     const unsigned m = __ballot_sync(0xffffffffu, odd);
     int at = 0;
     if (lane == 0) at = atomicAdd(&qcount, __popc(m));
@@ -1796,23 +1821,46 @@ smac_status predict_vstar(const char* fn, const smac_grid_desc* d, const smac_bo
     A.st[k][2] = (int)(S0 * S1);
   }
   fill_table(&A.bc, bc);
+  const dim3 block(32, 8);
+  const cudaStream_t cs = (cudaStream_t)stream;
+  const int wx = (d->nx + 1 + 31) / 32, wy = (d->ny + 1 + PV_Y - 1) / PV_Y, planes = d->nz + 1;
+  const int tx = (d->nx + 1 + PV_X - 1) / PV_X;
+  // One thread per face on grids too thin for the march, and where that is fewer
+  // than PF_WAVES waves of resident warps (more where the march has more tiles
+  // of a row: 31 faces against 32): a block of the march stages types, marches
+  // and empties its queue one after the other, and on a small grid that chain
+  // is the time.  Per face against march, us (plain; two-way with 20 spheres):
+  // 20^3 9.7, 19.2; 12.6, 26.9.  48^3 26, 38; 38, 53.  64^3 (6.4 waves) 46, 60;
+  // 70, 97.  160 x 90 x 24 (6.9) 55, 65; 73, 84.  24 x 90 x 160 (7.4) 83, 67;
+  // 102, 94.  94 x 80 x 60 (7.5, 4 tiles against 3) 78, 78; 109, 120.  72^3
+  // (8.1) 77, 73; 120, 115.  93 x 93 x 61 (8.9, 4 against 3) 94, 87; 129, 128.
+  // 96^3 158, 138; 215, 207.  192^3 1011, 681; 1271, 1028.
+  const long long warps = 3LL * wx * (d->ny + 1) * planes;
+  const bool thin = d->nx < 4 || d->ny < 4 || d->nz < 4;
+  const unsigned fz = 6u * (unsigned)((planes + 1) / 2);
+  if ((thin || 2 * wx * warps < (long long)(wx + tx) * PF_WAVES * PF_BLOCKS * 8 * sm_count()) && fz <= 65535u) {
+    const dim3 grid((unsigned)wx, (unsigned)wy, fz);
+    if (tw)
+      k_predict_faces<true><<<grid, block, 0, cs>>>(A);
+    else
+      k_predict_faces<false><<<grid, block, 0, cs>>>(A);
+    return launch_status(fn);
+  }
   // planes per chunk: the fewest steps per resident block, counting a chunk's
   // types, first side and first loads as three more
-  const int tx = (d->nx + 1 + PV_X - 1) / PV_X, ty = (d->ny + 1 + PV_Y - 1) / PV_Y, planes = d->nz + 1;
   const long long slots = (long long)PV_BLOCKS * sm_count();
   int zc = 1;
   long long best = -1;
   for (int cand = std::min(PV_ZMAX, planes); cand >= std::min(3, planes); --cand) {
-    const long long blocks = 3LL * tx * ty * ((planes + cand - 1) / cand);
+    const long long blocks = 3LL * tx * wy * ((planes + cand - 1) / cand);
     const long long cost = ((blocks + slots - 1) / slots) * (cand + 3);
     if (best < 0 || cost < best) { best = cost; zc = cand; }
   }
-  const dim3 grid((unsigned)tx, (unsigned)ty, 3u * (unsigned)((planes + zc - 1) / zc)), block(32, PV_Y);
-  const int fast = d->nx >= 4 && d->ny >= 4 && d->nz >= 4;
+  const dim3 grid((unsigned)tx, (unsigned)wy, 3u * (unsigned)((planes + zc - 1) / zc));
   if (tw)
-    k_predict_vstar<true><<<grid, block, 0, (cudaStream_t)stream>>>(A, zc, fast);
+    k_predict_march<true><<<grid, block, 0, cs>>>(A, zc, !thin);
   else
-    k_predict_vstar<false><<<grid, block, 0, (cudaStream_t)stream>>>(A, zc, fast);
+    k_predict_march<false><<<grid, block, 0, cs>>>(A, zc, !thin);
   return launch_status(fn);
 }
 
