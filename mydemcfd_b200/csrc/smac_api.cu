@@ -914,9 +914,13 @@ void setup_zm(smac_handle* h) {
 // rank of its two children: the first chunk is the planes per rank rounded
 // up to a multiple of 2^(z-coarsenings below it within the spread grids and
 // into the first held one).
+// The kernel's shared-memory limit belongs to the device and not to a handle:
+// every handle raises it to the device's most, so that none lowers it below
+// what another one's launches ask for.
 template <class T>
-bool cluster_attr(int bytes) {
-  if (cudaFuncSetAttribute(k_coarse_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
+bool cluster_fits(int bytes, int smem_optin) {
+  if (cudaFuncSetAttribute(k_coarse_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin) !=
+      cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -963,7 +967,7 @@ bool plan_cluster(smac_handle* h, int lk, int smem_optin) {
   }
   // (FP64 at 32^3 leaves no room for the residuals)
   P.scratch = (tot + cells + 3) * (int)sizeof(T) <= smem_optin ? take(cells) : -1;
-  if (!cluster_attr<T>((int)(tot * (int)sizeof(T)))) return false;
+  if (!cluster_fits<T>((int)(tot * (int)sizeof(T)), smem_optin)) return false;
   P.elems = (int)tot;
   P.nd = nd;
   P.lk = lk;
