@@ -1460,10 +1460,10 @@ smac_status run_solve(smac_handle* h, const double** xout) {
   int per_launch = 0;
   const double per_bytes = iteration_bytes(h, mixed, gmg, &per_launch);
   int restarts = 0;
-  int launched = 0;
-  const int max_launches = o.max_iter + 8;
+  int total = 0;     // iterations launched
+  int launched = 0;  // without those that found the solve stopped: what counts against max_iter
   for (;;) {
-    if (launched > max_launches) {  // the device sets done by max_iter; this is a second bound
+    if (launched - 8 > o.max_iter) {  // the device sets done by max_iter; this is a second bound
       set_err("run_solve: iteration bound exceeded without a device decision");
       return SMAC_NOT_CONVERGED;
     }
@@ -1474,13 +1474,16 @@ smac_status run_solve(smac_handle* h, const double** xout) {
     // ones an eighth of those done (one graph in a multigrid solve; a Jacobi
     // solve of hundreds of iterations used to wait after every second one).
     // Projection of 32^3 FP64 548 -> 542 us, 64^3 mixed 764 -> 758.
-    const int batch = launched == 0 ? (o.stop_rule == SMAC_STOP_RELATIVE && o.tol <= 1e-4 && o.max_iter >= 4 ? 2 : 1)
-                                    : std::max(1, launched / 16);
+    int batch = launched == 0 ? (o.stop_rule == SMAC_STOP_RELATIVE && o.tol <= 1e-4 && o.max_iter >= 4 ? 2 : 1)
+                              : std::max(1, launched / 16);
+    batch = std::min(batch, std::max(1, (o.max_iter - launched + 1) / 2));
     for (int q = 0; q < batch; ++q) CK(cudaGraphLaunch(ex, h->stream));
     launched += 2 * batch;
+    total += 2 * batch;
     TRY(scalars_to_host(h));
     CK(cudaStreamSynchronize(h->stream));
     if (h->hs->done) {
+      launched = h->hs->iter;
       if (h->hs->status == 2 && restarts < 3) {
         // Breakdown (p.Ap or r.z <= 0).  Near the rounding floor of a tight
         // tolerance it means the Krylov space is exhausted, not failure:
@@ -1562,7 +1565,7 @@ smac_status run_solve(smac_handle* h, const double** xout) {
   {
     const int it = h->hs->iter;
     h->alg_bytes += per_bytes * it;
-    h->launches += per_launch * launched;
+    h->launches += per_launch * total;
     if (mixed) {
       h->alg_bytes += (double)h->hs->reliable_count * (8 + 4 + 3 * 8 + 8 + 8 + 4) * (double)g.cells();
     }

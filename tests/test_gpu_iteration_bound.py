@@ -1,0 +1,37 @@
+"""How many iterations a solve may launch."""
+import dataclasses
+
+import pytest
+
+from mydemcfd_b200 import _native as nat
+from mydemcfd_b200 import workloads as W
+from mydemcfd_b200.solver import B200PressureSolver, DeviceGrid
+
+pytestmark = pytest.mark.gpu
+
+
+def make(n, ratio, **options):
+    case = dataclasses.replace(W.vof_case(n, seed=5, ratio=ratio), h=(1.0 / n,) * 3)
+    g = DeviceGrid.from_case(case)
+    s = B200PressureSolver(case.N, case.h, **options)
+    s.set_coefficients(g)
+    s.divergence(g, case.dt)
+    return g, s
+
+
+@pytest.mark.parametrize("n", [48, 64])
+def test_a_restarted_solve_may_use_every_iteration_it_is_allowed(n):
+    """A Jacobi solve of hundreds of iterations to 1e-14, whose recursive residual gets there before the true one, so
+    that PCG starts again: iterations launched after the first stop, which do nothing, do not count against
+    max_iter."""
+    g, s = make(n, 1000.0, solver_type=nat.PURENEUMANN_STANDARD_PCG, tol=1e-14, max_iter=100000)
+    its = s.solve_rhs(g.p_delta_)["iterations"]
+    assert its > 200
+    for extra in (0, 1, 2, 7):
+        s.set_options(max_iter=its + extra)
+        st = s.solve_rhs(g.p_delta_)
+        assert st["status"] == 0 and st["iterations"] == its and st["rel_residual"] <= 1e-14, (extra, st)
+    s.set_options(max_iter=its // 2)
+    st = s.solve_rhs(g.p_delta_, raise_on_fail=False)
+    assert st["status"] == nat.NOT_CONVERGED and st["iterations"] == its // 2, st
+    assert 1e-14 < st["rel_residual"] < 1e-4
