@@ -1469,13 +1469,13 @@ smac_status run_solve(smac_handle* h, const double** xout) {
     }
     // Launch a batch of iterations (one graph = two iterations); kernels after
     // convergence return at once.  The host waits for the flag after each
-    // batch, which leaves the GPU idle for some 7 us: the first batch has four
-    // iterations where the tolerance asks for more than two anyway, and later
-    // ones an eighth of those done (one graph in a multigrid solve; a Jacobi
-    // solve of hundreds of iterations used to wait after every second one).
-    // Projection of 32^3 FP64 548 -> 542 us, 64^3 mixed 764 -> 758.
-    int batch = launched == 0 ? (o.stop_rule == SMAC_STOP_RELATIVE && o.tol <= 1e-4 && o.max_iter >= 4 ? 2 : 1)
-                              : std::max(1, launched / 16);
+    // batch, which leaves the GPU idle for some 7 us: a batch is an eighth of
+    // the iterations done, one graph up to 32 of them.  Jacobi, FP64, one graph
+    // always: 32^3 (171 iterations) 4148 us, 64^3 (406) 11781, 128^3 (738)
+    // 63661; so 3816, 10466, 61434.  A first batch of four iterations would
+    // save one wait, and make a solve that set-up finds done (b = 0) take 175 us
+    // for 127 at 64^3.
+    int batch = std::max(1, launched / 16);
     batch = std::min(batch, std::max(1, (o.max_iter - launched + 1) / 2));
     for (int q = 0; q < batch; ++q) CK(cudaGraphLaunch(ex, h->stream));
     launched += 2 * batch;

@@ -1,4 +1,4 @@
-"""How many iterations a solve may launch."""
+"""How many iterations a solve may launch, and what it launches for nothing."""
 import dataclasses
 
 import pytest
@@ -35,3 +35,16 @@ def test_a_restarted_solve_may_use_every_iteration_it_is_allowed(n):
     st = s.solve_rhs(g.p_delta_, raise_on_fail=False)
     assert st["status"] == nat.NOT_CONVERGED and st["iterations"] == its // 2, st
     assert 1e-14 < st["rel_residual"] < 1e-4
+
+
+@pytest.mark.parametrize("precision", [nat.PRECISION_FP64, nat.PRECISION_MIXED])
+def test_a_zero_right_hand_side_launches_no_more_than_two_iterations(precision):
+    g, s = make(32, 100.0, precision=precision, tol=1e-8, max_iter=2)
+    capped = s.solve_rhs(g.p_delta_, raise_on_fail=False)
+    assert capped["iterations"] == 2
+    s.set_options(max_iter=2000)
+    g.rhs_.zero_()
+    s.set_rhs(g.rhs_)
+    st = s.solve_rhs(g.p_delta_)
+    assert st["status"] == 0 and st["iterations"] == 0 and not g.p_delta_.any()
+    assert st["kernel_launches"] <= capped["kernel_launches"]
