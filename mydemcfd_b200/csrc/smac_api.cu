@@ -93,6 +93,7 @@ void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cu
 }
 
 constexpr int MAXL = 16;
+static_assert(MAX_COARSE >= MAXL, "the single-CTA set may hold every grid");
 constexpr int COARSE_CELLS = 4096;  // grids at or below this size run in the single-CTA kernel
 
 enum CoefType { CT_F64 = 0, CT_F32 = 1, CT_BF16 = 2 };

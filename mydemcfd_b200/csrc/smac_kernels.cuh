@@ -1048,7 +1048,7 @@ struct CoarseLevel {
   void* x;
   void* rhs;
 };
-constexpr int MAX_COARSE = 8;
+constexpr int MAX_COARSE = 16;  // every grid of a hierarchy: 1024 x 2 x 2 has nine of at most 4096 cells
 struct CoarseSet {
   CoarseLevel L[MAX_COARSE];
   int n;  // grids in the set; L[0] receives rhs and returns x

@@ -75,3 +75,27 @@ def test_odd_extents_every_kernel_gives_the_same_bits(N, precision, outlet):
             assert np.array_equal(p, ref), options
         assert np.linalg.norm(p - ref) <= 1e-6 * np.linalg.norm(ref), options
         s.close()
+
+
+@pytest.mark.parametrize("precision", [nat.PRECISION_FP64, nat.PRECISION_MIXED])
+@pytest.mark.parametrize("N, min_coarse, levels", [
+    ((1024, 2, 2), 4, 9),    # 4096 cells, the most that one CTA takes, halved eight times
+    ((2, 801, 2), 4, 9),     # odd on the way down
+    ((3, 2, 640), 2, 10),    # 640, 320, ..., 5, 3, 2
+    ((257, 4, 3), 2, 9),
+])
+def test_one_cta_takes_as_many_grids_as_there_are(N, min_coarse, levels, precision):
+    """Long thin grids: more than eight grids of at most 4096 cells, solved twice."""
+    g, s, st = solved(N, precision, False, tol=1e-8, min_coarse=min_coarse)
+    assert s.num_levels() == levels and s.level_shape(levels - 1)[int(np.argmax(N))] <= 4
+    assert st["status"] == 0
+    first = g.p_delta_.clone()
+    s.divergence(g, 1.0)
+    s.solve_rhs(g.p_delta_)
+    assert torch.equal(first, g.p_delta_)
+    y = torch.zeros_like(g.rhs_)
+    s.apply_A(g.p_delta_, y)
+    b, ax = W.interior(g.rhs_.cpu().numpy()), W.interior(y.cpu().numpy())
+    b = b - b.mean()
+    slack = 1e-15 * 12 * N[0] ** 2 * np.linalg.norm(W.interior(g.p_delta_.cpu().numpy()))
+    assert np.linalg.norm(b - ax) <= 1e-8 * np.linalg.norm(b) + slack
