@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(TNT) k_setup_sum(Geom g, const double* __restr
 
 template <class TR>
 __global__ void __launch_bounds__(TNT) k_setup_project(Geom g, double* b, const uint8_t* __restrict__ fluid, TR* r,
-                                                       RedBuf red, Scalars* s, double tol, int kz) {
+                                                       RedBuf red, Scalars* s, int* host_done, double tol, int kz) {
   const int i = blockIdx.x * TBX + threadIdx.x;
   const int j = blockIdx.y * TBY + threadIdx.y;
   const int k0 = blockIdx.z * kz;
@@ -473,6 +473,7 @@ __global__ void __launch_bounds__(TNT) k_setup_project(Geom g, double* b, const 
       if (!isfinite(out[0])) { s->status = 3; s->done = 1; }
       else if (out[0] == 0.0) { s->done = 1; }  // b == 0: x = 0 is exact
       else if (s->stop_rule == 1 && out[1] < s->tol_max) { s->done = 1; }
+      if (s->done) *host_done = 1;  // (mapped; 0 otherwise, as the host left it)
     }
   }
 }
