@@ -1397,9 +1397,16 @@ smac_status smac_divergence(smac_handle* h, const double* vxs, const double* vys
   };
   constexpr std::true_type on{};
   constexpr std::false_type off{};
+  // Planes per thread: the more arrays, the fewer, as their loads' registers
+  // cost warps.  At 256^3: with both 307 us with one plane, 407 with two (taken
+  // past the launch limit of one only), 356 with loads at their use; void
+  // fractions 197 with two (273 at their use), surface tension 267 with two
+  // (299), plain 133 with four (135).
   constexpr std::integral_constant<int, 4> four{};
-  constexpr std::integral_constant<int, 2> two{};  // (more loads per plane)
-  if (eps && fsx) launch(two, on, on);
+  constexpr std::integral_constant<int, 2> two{};
+  constexpr std::integral_constant<int, 1> one{};
+  if (eps && fsx && g.nz <= 65535) launch(one, on, on);
+  else if (eps && fsx) launch(two, on, on);
   else if (eps) launch(two, on, off);
   else if (fsx) launch(two, off, on);
   else launch(four, off, off);

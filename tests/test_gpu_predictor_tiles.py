@@ -55,9 +55,9 @@ def test_marched_predictor_bit_exact_over_tile_edges(N, solid, two_way):
         assert np.array_equal(a, b), k
 
 
-def _device_us(fn):
+def _device_us(fn, stream=None):
     """Device time of one call of 20 in a graph."""
-    stream = torch.cuda.Stream()
+    stream = stream or torch.cuda.Stream()
     with torch.cuda.stream(stream):
         fn()
         stream.synchronize()
