@@ -583,25 +583,22 @@ __device__ __forceinline__ double st_diff(bool p, bool m, double fp, double f0, 
   return 0.0;
 }
 
-// Planes per thread of the two passes, whose loads are issued together: with
-// one, k_st_force took 113 us at 192^3, with two 97; the explicit half there
-// 1242, 1223, 1215 and 1228 us with one in the old form, one, two and four.
-constexpr int ST_KZ = 2;
-
 // Pass 1, k_calc_interface_normal (:87-182): grad alpha, |grad alpha| and the
 // unit normal of every C_INTERIOR cell; other cells are left as they are.
+// KZ planes per thread, their loads issued together.
+template <int KZ>
 __global__ void __launch_bounds__(256) k_st_normal(StArgs A) {
   const RefDims& R = A.R;
   const int ix = blockIdx.x * 32 + threadIdx.x + 1, iy = blockIdx.y * 8 + threadIdx.y + 1;
-  const int iz0 = blockIdx.z * ST_KZ + 1;
+  const int iz0 = blockIdx.z * KZ + 1;
   if (ix > R.Nx || iy > R.Ny) return;
   const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2), c0 = R.cell(ix, iy, iz0);
   const double* __restrict__ a = A.alpha;
   const uint8_t* __restrict__ ct = A.ct;
-  double az[ST_KZ + 2], ax[ST_KZ][2], ay[ST_KZ][2];
-  uint8_t tz[ST_KZ + 2], tx[ST_KZ][2], ty[ST_KZ][2];
+  double az[KZ + 2], ax[KZ][2], ay[KZ][2];
+  uint8_t tz[KZ + 2], tx[KZ][2], ty[KZ][2];
 #pragma unroll
-  for (int q = 0; q < ST_KZ + 2; ++q) {  // the own column, planes iz0 - 1 .. iz0 + KZ
+  for (int q = 0; q < KZ + 2; ++q) {  // the own column, planes iz0 - 1 .. iz0 + KZ
     az[q] = 0.0;
     tz[q] = 2;
     if (iz0 + q - 1 <= R.Nz + 1) {
@@ -610,7 +607,7 @@ __global__ void __launch_bounds__(256) k_st_normal(StArgs A) {
     }
   }
 #pragma unroll
-  for (int q = 0; q < ST_KZ; ++q) {
+  for (int q = 0; q < KZ; ++q) {
     const long long c = c0 + q * sxy;
     if (iz0 + q > R.Nz) break;
     ax[q][0] = a[c - 1];
@@ -623,7 +620,7 @@ __global__ void __launch_bounds__(256) k_st_normal(StArgs A) {
     ty[q][1] = ct[c + sx];
   }
 #pragma unroll
-  for (int q = 0; q < ST_KZ; ++q) {
+  for (int q = 0; q < KZ; ++q) {
     const long long c = c0 + q * sxy;
     if (iz0 + q > R.Nz) break;
     if (tz[q + 1] != kInterior) continue;
@@ -671,7 +668,7 @@ __device__ __forceinline__ double st_force(double sigma, double ap, double am, d
 
 constexpr int ST_TX = 32, ST_TY = 8;
 
-// Pass 2: curvature and face force fused.  A block owns a 32 x 8 tile of ST_KZ
+// Pass 2: curvature and face force fused.  A block owns a 32 x 8 tile of KZ
 // planes: each thread computes its cells' curvatures (stored) and the one
 // below the first, 40 threads per plane those of the tile's low-x column and
 // low-y row (into a shared tile), and after one barrier every thread writes
@@ -681,24 +678,25 @@ constexpr int ST_TX = 32, ST_TY = 8;
 // register, with a barrier per plane, took 2.5x as long.
 // Faces 1..N of every family are written (0 where the reference's memset
 // leaves 0); the rest is k_st_rim's.
+template <int KZ>
 __global__ void __launch_bounds__(ST_TX* ST_TY) k_st_force(StArgs A) {
-  __shared__ double ks[ST_KZ][ST_TY + 1][ST_TX + 1];
+  __shared__ double ks[KZ][ST_TY + 1][ST_TX + 1];
   const RefDims& R = A.R;
   const int tx = threadIdx.x, ty = threadIdx.y, t = ty * ST_TX + tx;
-  const int x0 = blockIdx.x * ST_TX, y0 = blockIdx.y * ST_TY, iz0 = blockIdx.z * ST_KZ + 1;
+  const int x0 = blockIdx.x * ST_TX, y0 = blockIdx.y * ST_TY, iz0 = blockIdx.z * KZ + 1;
   const int ix = x0 + tx + 1, iy = y0 + ty + 1;
   const bool in = ix <= R.Nx && iy <= R.Ny;
   const long long sx = R.Nx + 2, sxy = sx * (R.Ny + 2);
   const double* __restrict__ al = A.alpha;
   const uint8_t* __restrict__ ct = A.ct;
-  double k[ST_KZ], a[ST_KZ + 1], ax[ST_KZ], ay[ST_KZ], kb = 0.0;
-  bool fx[ST_KZ], fy[ST_KZ], fz[ST_KZ];
+  double k[KZ], a[KZ + 1], ax[KZ], ay[KZ], kb = 0.0;
+  bool fx[KZ], fy[KZ], fz[KZ];
   const long long c0 = in ? R.cell(ix, iy, iz0) : 0;
   if (in) {
     // everything the faces need but the shared tile, before the barrier
-    uint8_t tc[ST_KZ + 1], tl[ST_KZ][2];
+    uint8_t tc[KZ + 1], tl[KZ][2];
 #pragma unroll
-    for (int q = 0; q <= ST_KZ; ++q) {  // the own column, planes iz0 - 1 .. iz0 + KZ - 1
+    for (int q = 0; q <= KZ; ++q) {  // the own column, planes iz0 - 1 .. iz0 + KZ - 1
       a[q] = 0.0;
       tc[q] = 2;
       if (iz0 + q - 1 <= R.Nz) {
@@ -707,7 +705,7 @@ __global__ void __launch_bounds__(ST_TX* ST_TY) k_st_force(StArgs A) {
       }
     }
 #pragma unroll
-    for (int q = 0; q < ST_KZ; ++q) {
+    for (int q = 0; q < KZ; ++q) {
       const long long c = c0 + q * sxy;
       ax[q] = ay[q] = 0.0;
       tl[q][0] = tl[q][1] = 2;
@@ -719,7 +717,7 @@ __global__ void __launch_bounds__(ST_TX* ST_TY) k_st_force(StArgs A) {
       }
     }
 #pragma unroll
-    for (int q = 0; q < ST_KZ; ++q) {
+    for (int q = 0; q < KZ; ++q) {
       const bool i0 = tc[q + 1] == kInterior;
       fx[q] = ix >= 2 && i0 && tl[q][0] == kInterior;
       fy[q] = iy >= 2 && i0 && tl[q][1] == kInterior;
@@ -733,9 +731,9 @@ __global__ void __launch_bounds__(ST_TX* ST_TY) k_st_force(StArgs A) {
     if (fz[0]) kb = st_kappa(A, c0 - sxy, a[0]);
   }
 #pragma unroll
-  for (int q = 0; q < ST_KZ; ++q) ks[q][ty + 1][tx + 1] = in ? k[q] : 0.0;
+  for (int q = 0; q < KZ; ++q) ks[q][ty + 1][tx + 1] = in ? k[q] : 0.0;
   // the extra cells: column x0 (rows y0+1..y0+8) or row y0 (columns x0+1..x0+32) of each plane
-  for (int e = t; e < ST_KZ * (ST_TX + ST_TY); e += ST_TX * ST_TY) {
+  for (int e = t; e < KZ * (ST_TX + ST_TY); e += ST_TX * ST_TY) {
     const int q = e / (ST_TX + ST_TY), u = e - q * (ST_TX + ST_TY);
     const bool col = u < ST_TY;
     const int hx = col ? x0 : x0 + 1 + (u - ST_TY), hy = col ? y0 + 1 + u : y0;
@@ -750,7 +748,7 @@ __global__ void __launch_bounds__(ST_TX* ST_TY) k_st_force(StArgs A) {
   __syncthreads();
   if (!in) return;
 #pragma unroll
-  for (int q = 0; q < ST_KZ; ++q) {
+  for (int q = 0; q < KZ; ++q) {
     const int iz = iz0 + q;
     if (iz > R.Nz) break;
     const double kz = q ? k[q > 0 ? q - 1 : 0] : kb;
@@ -1757,9 +1755,23 @@ smac_status smac_surface_tension(const smac_grid_desc* d, const double* alpha, c
   cudaStream_t s = (cudaStream_t)stream;
   const unsigned bx = (unsigned)((d->nx + ST_TX - 1) / ST_TX), by = (unsigned)((d->ny + ST_TY - 1) / ST_TY);
   k_st_rim<<<dim3(64, 9), 256, 0, s>>>(A);
-  const unsigned bz = (unsigned)((d->nz + ST_KZ - 1) / ST_KZ);
-  k_st_normal<<<dim3(bx, by, bz), dim3(32, 8), 0, s>>>(A);
-  k_st_force<<<dim3(bx, by, bz), dim3(ST_TX, ST_TY), 0, s>>>(A);
+  const dim3 block(ST_TX, ST_TY);
+  const dim3 planes(bx, by, (unsigned)d->nz), pairs(bx, by, (unsigned)((d->nz + 1) / 2));
+  const bool flat = d->nz <= 65535;  // (a launch's planes)
+  // One plane per thread, in the second pass two from eight waves of its blocks
+  // on: a plane more is another chain of loads on a small grid, and fewer
+  // repeated curvatures on a large one.  us, planes in the first and second
+  // pass 1 and 1, 1 and 2, 2 and 2: 32^3 9.3, 12.1, 12.8; 64^3 13.3, 14.5, 14.6;
+  // 96^3 (4.7 waves) 24.5, 24.2, 24.5; 112^3 (8.5) 38.7, 38.1, 38.9; 192^3 180,
+  // 173, 178; 256^3 396, 380, 385.
+  if (flat)
+    k_st_normal<1><<<planes, block, 0, s>>>(A);
+  else
+    k_st_normal<2><<<pairs, block, 0, s>>>(A);
+  if (flat && (long long)bx * by * d->nz < 8LL * 5 * sm_count())
+    k_st_force<1><<<planes, block, 0, s>>>(A);
+  else
+    k_st_force<2><<<pairs, block, 0, s>>>(A);
   return launch_status(fn);
 }
 

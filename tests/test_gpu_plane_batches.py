@@ -5,7 +5,7 @@ import torch
 
 from _cases import ref_grid
 from mydemcfd_b200 import workloads as W
-from mydemcfd_b200.solver import B200PressureSolver, DeviceGrid
+from mydemcfd_b200.solver import B200PressureSolver, DeviceGrid, face_gradp_device, surface_tension_device
 from oracle import oracle as O
 from test_gpu_post import ST_KEYS, run_surface
 from test_gpu_predictor_tiles import _device_us
@@ -63,6 +63,16 @@ def test_surface_tension_bit_exact_over_depths(N):
             assert np.array_equal(a, b), k
 
 
+@pytest.mark.parametrize("N", [(33, 9, 1479), (33, 9, 1480), (33, 9, 1481),    # below eight waves of blocks, from them on
+                               (65, 5, 1975), (2, 2, 65537)])                  # beyond a launch's planes
+def test_surface_tension_bit_exact_with_two_planes(N):
+    n, h, alpha, ct, sigma = W.surface_case(N, seed=6, kind="random", solid_fraction=0.1 if min(N) > 4 else 0.0)
+    work = [rnd(900 + k, W.shapes(n)["cell"]) for k in range(5)]
+    for k, a, b in zip(ST_KEYS, run_surface(n, h, alpha, ct, sigma, work),
+                       O.surface_tension(n, h, alpha, ct, sigma, *work)):
+        assert np.array_equal(a, b), k
+
+
 @pytest.mark.parametrize("N", SIZES)
 def test_imported_operator_with_solids(N):
     """The operator of masked coefficients (solids, faces that are not F_INTERIOR, Dirichlet walls) against numpy;
@@ -118,3 +128,17 @@ def test_divergence_of_a_coupled_step_runs_near_the_plain_ones_bandwidth():
         us[key] = _device_us(lambda: s.divergence(g, 1.0), stream) / nbytes
     print(f"divergence 192^3: {41 * us['plain']:.1f} us, with everything {105 * us['coupled']:.1f} us")
     assert us["coupled"] <= us["plain"] / 0.9
+
+
+def test_surface_tension_of_a_small_grid_takes_one_plane_per_thread():
+    """32^3, against the one-load kernel of the pressure gradient: 5 times its device time; 6.5 and more with two
+    planes per thread, whose chains of loads run one after the other on a grid of one wave."""
+    n, h, alpha, ct, sigma = W.surface_case((32, 32, 32), seed=6, kind="sphere")
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    a, c = dev(alpha), dev(ct)
+    work = [torch.zeros_like(a) for _ in range(5)]
+    faces = [torch.zeros(W.shapes(n)[k], dtype=torch.float64, device="cuda") for k in "xyz"]
+    us = _device_us(lambda: surface_tension_device(n, h, a, c, sigma, work, faces))
+    gradp = _device_us(lambda: face_gradp_device(n, h, a, faces))
+    print(f"surface tension 32^3: {us:.1f} us, pressure gradient {gradp:.1f} us")
+    assert us <= 6.1 * gradp
