@@ -376,10 +376,9 @@ int zm_shape(const smac_handle* h, const Geom& g, bool automatic) {
 
 template <class T, int NV, int WX, int TY, int MODE, bool DOT>
 void launch_zm_shape(smac_handle* h, int l, const T* xin, T* xout, const T* rhs, const double* sh, const void* bx,
-                     const void* by, const void* bz, int c0, const T* xc, int ctas) {
+                     const void* by, const void* bz, int c0, int ctas) {
   constexpr int NT = ZmTile<T, NV, WX, TY, MODE>::NT;
   const Geom& g = h->lv[l].g;
-  const Level& Lc = h->lv[l + 1 < h->nlev ? l + 1 : l];
   // z-chunk: the fewest planes per CTA, counting the two extra c0 planes of each item
   const long long nty = (g.ny + TY - 1) / TY;
   const long long slots = (long long)ctas * h->num_sms;
@@ -407,14 +406,14 @@ void launch_zm_shape(smac_handle* h, int l, const T* xin, T* xout, const T* rhs,
   const uintptr_t al = (uintptr_t)xin | (uintptr_t)rhs | (uintptr_t)bx | (uintptr_t)by | (uintptr_t)bz;
   const int pf = ((al & 15u) == 0 && 5.0 * (double)g.alloc * sizeof(T) > (double)h->l2_bytes) ? SMAC_ZM_PF : 0;
   launch_pdl(k_rbgs_zm<T, NV, WX, TY, MODE, DOT>, G, NT, ZmTile<T, NV, WX, TY, MODE>::SMEM, h->stream, g, xin, xout,
-      rhs, sh, S, c0, xc, Lc.g, Lc.cx, Lc.cy, Lc.cz, h->s, h->red, zc, pf);
+      rhs, sh, S, c0, h->s, h->red, zc, pf);
 }
 
 template <class T, int MODE, bool DOT>
 void launch_zm(smac_handle* h, int l, int shape, const T* xin, T* xout, const T* rhs, const double* sh,
-               const void* bx, const void* by, const void* bz, int c0, const T* xc) {
+               const void* bx, const void* by, const void* bz, int c0) {
   const int n = h->zm_ctas[sizeof(T) == 8 ? 1 : 0][shape];
-#define ZM_SHAPE(S) launch_zm_shape<T, zm_nv<T>(S), zm_wx<T>(S), zm_ty<T>(S), MODE, DOT>(h, l, xin, xout, rhs, sh, bx, by, bz, c0, xc, n)
+#define ZM_SHAPE(S) launch_zm_shape<T, zm_nv<T>(S), zm_wx<T>(S), zm_ty<T>(S), MODE, DOT>(h, l, xin, xout, rhs, sh, bx, by, bz, c0, n)
   if (shape == 0) ZM_SHAPE(0);
   else if (shape == 1) ZM_SHAPE(1);
   else if (shape == 2) ZM_SHAPE(2);
@@ -426,12 +425,12 @@ void launch_zm(smac_handle* h, int l, int shape, const T* xin, T* xout, const T*
 #undef ZM_SHAPE
 }
 
+// mode 0 plain, 1 from zero (the prolongation is a pass of its own, k_prolong_add)
 template <class T>
 void launch_zm_any(smac_handle* h, int l, int zs, int mode, bool dot, const T* xin, T* xout, const T* rhs,
-                   const double* sh, const void* bx, const void* by, const void* bz, int c0, const T* xc) {
-  if (mode == 0) { if (dot) launch_zm<T, 0, true>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0, xc); else launch_zm<T, 0, false>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0, xc); }
-  else if (mode == 1) { if (dot) launch_zm<T, 1, true>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0, xc); else launch_zm<T, 1, false>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0, xc); }
-  else { if (dot) launch_zm<T, 2, true>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0, xc); else launch_zm<T, 2, false>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0, xc); }
+                   const double* sh, const void* bx, const void* by, const void* bz, int c0) {
+  if (mode == 0) { if (dot) launch_zm<T, 0, true>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0); else launch_zm<T, 0, false>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0); }
+  else { if (dot) launch_zm<T, 1, true>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0); else launch_zm<T, 1, false>(h, l, zs, xin, xout, rhs, sh, bx, by, bz, c0); }
 }
 
 // One fused red-black sweep of grid l (mode 0 plain, 1 from zero, 2 with the
@@ -459,10 +458,10 @@ bool launch_sweep(smac_handle* h, int l, int mode, bool dot, const T* xin, T* xo
         const int G = (int)std::max(1LL, std::min(8LL * h->num_sms, (vecs + 255) / 256));
         launch_pdl(k_prolong_add<T>, G, 256, 0, h->stream, g, const_cast<T*>(xin), xc, Lc.g, Lc.cx, Lc.cy, Lc.cz,
             h->s);
-        launch_zm_any<T>(h, l, zs, 0, dot, xin, xout, rhs, sh, bx, by, bz, c0, nullptr);
+        launch_zm_any<T>(h, l, zs, 0, dot, xin, xout, rhs, sh, bx, by, bz, c0);
         return true;
       }
-      launch_zm_any<T>(h, l, zs, mode, dot, xin, xout, rhs, sh, bx, by, bz, c0, xc);
+      launch_zm_any<T>(h, l, zs, mode, dot, xin, xout, rhs, sh, bx, by, bz, c0);
       return false;
     }
     const bool ok = sizeof(T) == 8 ? L.tma64 : L.tma32;
@@ -870,7 +869,7 @@ cudaError_t tma_attr() {
 
 // Resident CTAs per SM of each z-march shape (0: not usable): the kernels'
 // shared-memory limit raised to their needs, then the fewest resident CTAs
-// of the six forms.
+// of the four forms.
 template <class T, int SH, int MODE, bool DOT>
 int zm_occupancy_one() {
   constexpr int NV = zm_nv<T>(SH), WX = zm_wx<T>(SH), TY = zm_ty<T>(SH);
@@ -887,12 +886,8 @@ int zm_occupancy_one() {
 }
 template <class T, int SH>
 int zm_occupancy() {
-  const int n[6] = {zm_occupancy_one<T, SH, 0, false>(), zm_occupancy_one<T, SH, 0, true>(),
-                    zm_occupancy_one<T, SH, 1, false>(), zm_occupancy_one<T, SH, 1, true>(),
-                    zm_occupancy_one<T, SH, 2, false>(), zm_occupancy_one<T, SH, 2, true>()};
-  int m = n[0];
-  for (int v : n) m = std::min(m, v);
-  return m;
+  return std::min(std::min(zm_occupancy_one<T, SH, 0, false>(), zm_occupancy_one<T, SH, 0, true>()),
+                  std::min(zm_occupancy_one<T, SH, 1, false>(), zm_occupancy_one<T, SH, 1, true>()));
 }
 void setup_zm(smac_handle* h) {
   h->zm_ctas[0][0] = zm_occupancy<float, 0>();
@@ -1515,7 +1510,7 @@ smac_status run_solve(smac_handle* h, const double** xout) {
         const int it_now = hs0.iter;
         auto S = stencil<double, double>(g, h->lv[0].bx64, h->lv[0].by64, h->lv[0].bz64);
         if (mixed) {
-          // fold the FP32 increment into x64 and recompute r (k_reliable
+          // fold the FP32 increment into x64 and recompute r (k_reliable_vec
           // decides convergence on the true residual)
           h->hs->done = 0;
           h->hs->status = 0;

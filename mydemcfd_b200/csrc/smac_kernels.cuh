@@ -762,21 +762,6 @@ __global__ void __launch_bounds__(TNT) k_dot_rz(Geom g, const T* __restrict__ r,
   }
 }
 
-// d = z + beta d
-template <class T>
-__global__ void __launch_bounds__(TNT) k_dir(Geom g, const T* __restrict__ z, T* d, const Scalars* s, int kz) {
-  if (s->done) return;
-  const int i = blockIdx.x * TBX + threadIdx.x;
-  const int j = blockIdx.y * TBY + threadIdx.y;
-  const int k0 = blockIdx.z * kz;
-  const T beta = (T)s->beta;
-  if (i < g.nx && j < g.ny) {
-    const int k1 = min(k0 + kz, g.nz);
-    int c = g.idx(i, j, k0);
-    for (int k = k0; k < k1; ++k, c += g.ps) d[c] = z[c] + beta * d[c];
-  }
-}
-
 // FP64 true residual r = b - A x with statistics (final check, plain mode).
 // When `restart` is set and the test fails, r is overwritten with the true
 // residual and PCG restarts from it.

@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(DMV_TX * DMV_TY) k_dir_matvec_vec(Geom g, cons
       A xcm[NV];
 #pragma unroll
       for (int e = 0; e < NV; ++e) xcm[e] = (fl[e] & 2) ? xc[e] : (A)0;
-      // x-neighbours across the vector edge (the unmasked D, as k_dir_matvec reads them)
+      // x-neighbours across the vector edge (the unmasked D)
       A left = __shfl_up_sync(0xffffffffu, xc[NV - 1], 1);
       A right = __shfl_down_sync(0xffffffffu, xc[0], 1);
       T bxr = __shfl_down_sync(0xffffffffu, bxs[0], 1);

@@ -130,7 +130,6 @@ template <class T, int NV>
 struct ZmOps {
   typename VecN<T, NV>::type rh, bx, by, byu, bzu, x1, xo;
   T bxe;
-  T c1[2];  // with the prolongation on a grid halved in every direction: the parents of x1
 };
 // Operands of the colour-(1-c0) pass on plane m, carried to the next step:
 // per cell of that colour its rhs and six weights.
@@ -142,8 +141,7 @@ struct ZmBlk {
 template <class T, int NV_, int WX, int TY, int MODE, bool DOT>
 __global__ void __launch_bounds__(ZmTile<T, NV_, WX, TY, MODE>::NT, ZmTile<T, NV_, WX, TY, MODE>::MINB)
     k_rbgs_zm(Geom g, const T* __restrict__ xin, T* __restrict__ xout, const T* __restrict__ rhs, const double* shift,
-              Stencil<T, T> S, int c0, const T* __restrict__ xc, Geom gc, int cx, int cy, int cz, Scalars* s,
-              RedBuf red, int zchunk, int pf) {
+              Stencil<T, T> S, int c0, Scalars* s, RedBuf red, int zchunk, int pf) {
   pdl_enter();
   typedef ZmTile<T, NV_, WX, TY, MODE> L;
   typedef typename VecN<T, NV_>::type V;
@@ -211,50 +209,15 @@ __global__ void __launch_bounds__(ZmTile<T, NV_, WX, TY, MODE>::NT, ZmTile<T, NV
     const int jo = wr == 0 ? j - 1 : j + 1;  // ring warps: the row beyond the ring
     const bool jo_ok = ring && jo >= 0 && jo < g.ny;
 
-    // the input vector of plane m, row jj (the coarse correction added in MODE 2); 0 outside the grid
+    // the input vector of plane m, row jj; 0 outside the grid
     auto load_x = [&](int m, int jj, bool ok) -> V {
       if constexpr (MODE == 1) return zero();
       if (!ok || !col_ok || m < 0 || m >= g.nz) return zero();
-      V v = *reinterpret_cast<const V*>(xin + g.idx(ib, jj, m));
-      if constexpr (MODE == 2) {
-        T* pv = reinterpret_cast<T*>(&v);
-#pragma unroll
-        for (int e = 0; e < NV; ++e) {
-          const int i = ib + e;
-          if (i < g.nx) pv[e] = (T)Ar<A>::add((A)pv[e], (A)xc[gc.idx(cx ? i >> 1 : i, cy ? jj >> 1 : jj, cz ? m >> 1 : m)]);
-        }
-      }
-      return v;
+      return *reinterpret_cast<const V*>(xin + g.idx(ib, jj, m));
     };
     auto load_v = [&](const T* a, int m, int jj, bool ok) -> V {
       if (!ok || !col_ok) return zero();
       return *reinterpret_cast<const V*>(a + g.idx(ib, jj, m));
-    };
-    // With the prolongation on a grid halved in every direction, the input
-    // vector of the lane's row is loaded as it is and its cells' parents
-    // (NV/2 coarse values) beside it; the sum is formed when the vector is
-    // used, a step later, so that no load is waited for where it is issued.
-    // (The ring rows' row beyond takes the immediate path: those warps wait
-    // at the step's barrier anyway.)
-    const bool pro4 = MODE == 2 && cx && cy && cz;
-    auto load_parents = [&](int m, int jj, bool ok, T (&c)[2]) {
-      c[0] = c[1] = (T)0;
-      if (!ok || !col_ok || m < 0 || m >= g.nz || ib >= g.nx) return;
-      const T* p = xc + gc.idx(ib >> 1, jj >> 1, m >> 1);
-      if constexpr (NV == 4) {
-        const typename Vec2<T>::type v = *reinterpret_cast<const typename Vec2<T>::type*>(p);
-        c[0] = v.x;
-        c[1] = v.y;
-      } else {
-        c[0] = p[0];
-      }
-    };
-    auto add_parents = [&](V v, const T (&c)[2]) -> V {
-      T* pv = reinterpret_cast<T*>(&v);
-#pragma unroll
-      for (int e = 0; e < NV; ++e)
-        if (ib + e < g.nx) pv[e] = (T)Ar<A>::add((A)pv[e], (A)c[e >> 1]);
-      return v;
     };
     auto load_ops = [&](int m, Ops& o) {
       const bool ok = row_ok && m >= 0 && m < g.nz;
@@ -264,15 +227,8 @@ __global__ void __launch_bounds__(ZmTile<T, NV_, WX, TY, MODE>::NT, ZmTile<T, NV
       o.by = load_v(S.by, m, j, ok);
       o.byu = load_v(S.by, m, j + 1, ok);
       o.bzu = load_v(S.bz, m + 1, j, row_ok && m + 1 >= 0 && m + 1 <= g.nz);  // z-face m+1 (0..nz)
-      if (pro4) {
-        o.x1 = (row_ok && col_ok && m + 1 >= 0 && m + 1 < g.nz) ? *reinterpret_cast<const V*>(xin + g.idx(ib, j, m + 1))
-                                                                : zero();
-        o.xo = load_x(m, jo, jo_ok);
-        load_parents(m + 1, j, row_ok, o.c1);
-      } else {
-        o.x1 = load_x(m + 1, j, row_ok);
-        o.xo = load_x(m, jo, jo_ok);
-      }
+      o.x1 = load_x(m + 1, j, row_ok);
+      o.xo = load_x(m, jo, jo_ok);
     };
 
     // The rows the tile reads on one plane (j0-2 .. j0+TY+1, clipped to the
@@ -328,7 +284,6 @@ __global__ void __launch_bounds__(ZmTile<T, NV_, WX, TY, MODE>::NT, ZmTile<T, NV
       const V bz_c = nxt.bzu;  // z-faces k (the previous step's faces k-1+1), read before nxt is reloaded
       if (k + 1 <= z1) load_ops(k + 1, nxt);
       if (pf > 0 && k + 1 + pf <= z1) prefetch(k + 1 + pf);
-      if (pro4) cur.x1 = add_parents(cur.x1, cur.c1);  // the deferred prolongation of this step's input
       // --- the input of plane k+1 becomes visible to the rows above and below
       *reinterpret_cast<V*>(Mrow(k + 1, wr) + ib) = cur.x1;
       T xh_p[H];
