@@ -48,3 +48,19 @@ def test_a_zero_right_hand_side_launches_no_more_than_two_iterations(precision):
     st = s.solve_rhs(g.p_delta_)
     assert st["status"] == 0 and st["iterations"] == 0 and not g.p_delta_.any()
     assert st["kernel_launches"] <= capped["kernel_launches"]
+
+
+@pytest.mark.parametrize("precision", [nat.PRECISION_FP64, nat.PRECISION_MIXED])
+def test_a_long_solve_runs_in_batches(precision):
+    """A Jacobi solve of hundreds of iterations: batches of an eighth of those done find the same end as a solve that
+    may launch no more than it needs, and the mixed form takes about the iterations of FP64."""
+    g, s = make(64, 1000.0, solver_type=nat.PURENEUMANN_STANDARD_PCG, precision=precision, tol=1e-10)
+    st = s.solve_rhs(g.p_delta_)
+    assert st["status"] == 0 and st["rel_residual"] <= 1e-10
+    assert 500 < st["iterations"] < 600      # 547 in FP64, 572 mixed
+    p = g.p_delta_.clone()
+    s.set_options(max_iter=st["iterations"])
+    s.divergence(g, 1.0)
+    again = s.solve_rhs(g.p_delta_)
+    assert again["iterations"] == st["iterations"] and (p == g.p_delta_).all()
+    assert again["kernel_launches"] <= st["kernel_launches"]
