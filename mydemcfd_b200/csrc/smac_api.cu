@@ -190,12 +190,10 @@ T* base_of(const Geom& g, T* p) {
 }
 
 // Planes per block of a kernel that marches in z with bx x by blocks per
-// plane: as many as leave MARCH_BLOCKS blocks (of 128 threads) per SM.  The
-// direction kernel at 64^3 (FP32), 64 blocks of 16 planes, took 26 us.  With
-// no such bound, 4, 8, 16 and 32 blocks: mixed projection of 64^3 908, 822,
-// 821, 822, 822 us, of 150 x 100 x 75 1686, 1558, 1581, 1614, 1600; pressure
-// step of 192^3 6664, 6661, 6556, 6561, 6720; projection of 256^3 5746, 5748,
-// 5752, 5777, 5856.
+// plane: 16 on deep grids, halved until there are MARCH_BLOCKS blocks (of 128
+// threads) per SM.  Mixed projection of 64^3 908 us without the halving, 821
+// with it.  Half as many blocks cost the pressure step of 192^3 2%, four times
+// as many that of 192^3 and the projection of 256^3 2%.
 constexpr int MARCH_BLOCKS = 8;
 inline int march_kz(const smac_handle* h, const Geom& g, long long bx, long long by, int least) {
   int kz = g.nz >= 64 ? 16 : (g.nz >= 16 ? 8 : 4);
@@ -385,12 +383,10 @@ void launch_zm_shape(smac_handle* h, int l, const T* xin, T* xout, const T* rhs,
   int zc = g.nz;
   long long best = -1;
   // (an item costs about six steps beyond its planes: two extra c0 planes and
-  // the exposed latency of its first loads; measured at 192^3 and 256^3)
-  // Down to one plane: a grid too small for an item per CTA then ends in the
-  // fewest steps (with at least four planes an item, 64^3 had 176 items for
-  // 444 CTAs; projections of 32^3 FP64, 64^3, 150 x 100 x 75 and 256^3 mixed
-  // took 615, 796, 1581 and 5727 us, 572, 770, 1524 and 5680 with two, 553,
-  // 770, 1528 and 5679 with one).
+  // the exposed latency of its first loads; measured at 192^3 and 256^3).  Down
+  // to one plane: a grid too small for an item per CTA then ends in the fewest
+  // steps.  Projection with at least four planes an item, two, one: 32^3 FP64
+  // 615, 572, 553 us, 256^3 mixed 5727, 5680, 5679.
   for (int cand = std::min(64, g.nz); cand >= 1; --cand) {
     const long long items = nty * ((g.nz + cand - 1) / cand);
     const long long cost = ((items + slots - 1) / slots) * (cand + 6);
@@ -1105,9 +1101,9 @@ smac_status smac_create(const smac_grid_desc* desc, const smac_options* opts, vo
   };
   // hierarchy: halve a direction while the result stays >= min_coarse, an odd
   // extent n to (n + 1) / 2 (k_coarsen_coeffs).  Stopping a direction at its
-  // first odd extent left a coarsest grid of up to the whole problem to one
-  // CTA and a few sweeps: 150 x 100 x 75 took 58 iterations and 120 ms,
-  // 99^3 64 and 848 ms (mixed).
+  // first odd extent leaves a coarsest grid of up to the whole problem to one
+  // CTA and a few sweeps: 150 x 100 x 75, mixed, 59 iterations and 125 ms, 7 and
+  // 1.5 ms so.
   {
     int nx = desc->nx, ny = desc->ny, nz = desc->nz;
     double ix2 = 1.0 / (desc->dx * desc->dx), iy2 = 1.0 / (desc->dy * desc->dy), iz2 = 1.0 / (desc->dz * desc->dz);

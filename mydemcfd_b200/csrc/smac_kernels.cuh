@@ -39,10 +39,9 @@ constexpr int TNT = TBX * TBY;
 // Also the FP32 weights of the mixed form (m*), the cell bits (bit 0
 // C_INTERIOR, bit 1 fluid: C_INTERIOR with a non-zero diagonal, the cells that
 // carry unknowns) and the number of fluid cells.  One pass: a thread holds the
-// six masked f_b of its cell and marches in z.  (Import, count and FP32
-// conversions used to be five launches here, and four to seven per coarse
-// grid: smac_set_coefficients took 145, 173, 269, 432 and 765 us at 32^3,
-// 64^3, 128^3, 192^3 and 256^3; 66, 73, 158, 310 and 574 now.)
+// six masked f_b of its cell and marches in z.  (smac_set_coefficients takes
+// 66, 158 and 574 us at 32^3, 128^3 and 256^3; 145, 269 and 765 with the
+// import, the count and each conversion as launches of their own.)
 __global__ void __launch_bounds__(TNT) k_import_coeffs(
     Geom g, RefDims R, const double* __restrict__ fbx, const double* __restrict__ fby, const double* __restrict__ fbz,
     const uint8_t* __restrict__ ct, const uint8_t* __restrict__ fxt, const uint8_t* __restrict__ fyt,
